@@ -102,6 +102,7 @@ struct Engine {
     int device = 0;
     int smCount = 148;
     cudaStream_t stream = nullptr;
+    SideStream side;               // kernels beside those of `stream`, joined before the stage ends
     int precision = DSMC_PRECISION_FP64;
     DsmcCaseParams params{};
     DsmcMeshMessage mess{};
@@ -196,6 +197,9 @@ struct Engine {
         }
         for (void* p : allocs) cudaFree(p);
         allocs.clear();
+        if (side.forked) { cudaEventDestroy(side.forked); side.forked = nullptr; }
+        if (side.joined) { cudaEventDestroy(side.joined); side.joined = nullptr; }
+        if (side.stream) { cudaStreamDestroy(side.stream); side.stream = nullptr; }
         if (stream) { cudaStreamDestroy(stream); stream = nullptr; }
     }
 
@@ -422,7 +426,13 @@ struct Engine {
         }
         cudaDeviceGetAttribute(&smCount, cudaDevAttrMultiProcessorCount, device);
         shape.smCount = smCount;
-        if (!cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
+        int least = 0, greatest = 0;
+        if (!cuda(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
+            !cuda(cudaDeviceGetStreamPriorityRange(&least, &greatest), "stream priorities") ||
+            !cuda(cudaStreamCreateWithPriority(&side.stream, cudaStreamNonBlocking, greatest), "cudaStreamCreate") ||
+            !cuda(cudaEventCreateWithFlags(&side.forked, cudaEventDisableTiming), "cudaEventCreate") ||
+            !cuda(cudaEventCreateWithFlags(&side.joined, cudaEventDisableTiming), "cudaEventCreate"))
+            return false;
         ncell = md->ncell;
         nface = md->nface;
         npoint = md->npoint;
@@ -1070,7 +1080,7 @@ struct Engine {
         if (sort) {
             b.A = a.B; b.B = a.A; b.startA = a.startB; b.startB = const_cast<int*>(a.startA);
         }
-        if (coll) launch_collide<Real>(b, shape, stream);
+        if (coll) launch_collide<Real>(b, shape, stream, side);
         if (events) cudaEventRecord(ev[4], stream);
         if (samp) launch_sample<Real>(b, false, shape, stream);
         if (events) cudaEventRecord(ev[5], stream);

@@ -893,43 +893,45 @@ __device__ __forceinline__ PairDraw pair_draw(int c, int istep, int j, int n, co
 __device__ __forceinline__ double psqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float psqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 
+// A particle's collision state: velocity and internal energy.
+template <typename Real>
+struct PState {
+    Real x, y, z, i;
+};
+
 // collisionVelocity, src/ProcessDSMC.cpp:2679-2744, on one candidate pair,
 // in two halves: the acceptance test (pair_accept) and, for an accepted
 // pair, the post-collision state (pair_execute). pair_execute recomputes the
 // relative velocity from the same stored velocities, so the halves give the
-// bits of the one-piece test-and-collide. Particle k of the cell is at
-// vx[k * stride] (and likewise vy, vz, ir). w2, w3: words 2 and 3 of the
-// pair's block 0. The FP64 branch rounds each operation on its own in the
-// reference's evaluation order; the FP32 branch lets the compiler fuse.
+// bits of the one-piece test-and-collide. w2, w3: words 2 and 3 of the
+// pair's block 0; cr: the relative speed, for the cell's crmax. The FP64
+// branch rounds each operation on its own in the reference's evaluation
+// order; the FP32 branch lets the compiler fuse.
 template <typename Real>
-__device__ __forceinline__ bool pair_accept(const Real* vx, const Real* vy, const Real* vz, int stride, int k1,
-                                            int k2, uint32_t w2, uint32_t w3, const DevConsts& C, double consCrm,
-                                            Real crm0, Real& crmLocal)
+__device__ __forceinline__ bool pair_accept(const PState<Real>& p, const PState<Real>& q, uint32_t w2, uint32_t w3,
+                                            const DevConsts& C, double consCrm, Real crm0, bool splitSum, Real& cr)
 {
-    k1 *= stride;
-    k2 *= stride;
     if constexpr (sizeof(Real) == 8) {
-        const double vr0 = ds(vx[k1], vx[k2]), vr1 = ds(vy[k1], vy[k2]), vr2 = ds(vz[k1], vz[k2]);
-        const double cr = sqrt(da(da(dm(vr0, vr0), dm(vr1, vr1)), dm(vr2, vr2)));
-        if (cr > crmLocal) crmLocal = cr;
+        const double vr0 = ds(p.x, q.x), vr1 = ds(p.y, q.y), vr2 = ds(p.z, q.z);
+        cr = sqrt(da(da(dm(vr0, vr0), dm(vr1, vr1)), dm(vr2, vr2)));
         const double accept = dd(collision_diameter(dm(cr, C.vrms), C.cdPrefactor, C.eta), consCrm);
         return unit64(w2, w3) < accept;
     } else {
-        const float vr0 = vx[k1] - vx[k2], vr1 = vy[k1] - vy[k2], vr2 = vz[k1] - vz[k2];
-        const float cr = psqrt(vr0 * vr0 + vr1 * vr1 + vr2 * vr2);
-        if (cr > crmLocal) crmLocal = cr;
+        const float vr0 = p.x - q.x, vr1 = p.y - q.y, vr2 = p.z - q.z;
+        // the squares added in one rounding each; in cells whose pairs ran
+        // in place or alone (splitSum) the last one is rounded on its own
+        const float xy = fmaf(vr0, vr0, __fmul_rn(vr1, vr1));
+        cr = psqrt(splitSum ? __fadd_rn(xy, __fmul_rn(vr2, vr2)) : fmaf(vr2, vr2, xy));
         // ratio of the VHS sigma*c at cr and at crmax: (cr/crmax)^(1-2 eta)
         const float accept = exp2f(C.vhsExpF * __log2f(__fdividef(cr, crm0)));
         return unit32(w2) < accept;
     }
 }
 
-__device__ __forceinline__ void pair_execute_fp64(double* vx, double* vy, double* vz, double* ir, int k1, int k2,
-                                                  const PairDraw& d, const DevConsts& C)
+__device__ __forceinline__ void pair_execute_fp64(PState<double>& p, PState<double>& q, const PairDraw& d,
+                                                  const DevConsts& C)
 {
-    const double v1x = vx[k1], v1y = vy[k1], v1z = vz[k1];
-    const double v2x = vx[k2], v2y = vy[k2], v2z = vz[k2];
-    const double vr0 = ds(v1x, v2x), vr1 = ds(v1y, v2y), vr2 = ds(v1z, v2z);
+    const double vr0 = ds(p.x, q.x), vr1 = ds(p.y, q.y), vr2 = ds(p.z, q.z);
     const double cr2 = da(da(dm(vr0, vr0), dm(vr1, vr1)), dm(vr2, vr2));
     const double cr = sqrt(cr2);
     double preErt = dm(0.25, cr2);
@@ -939,16 +941,16 @@ __device__ __forceinline__ void pair_execute_fp64(double* vx, double* vy, double
     const double rChi = unit64(b3.x, b3.y), th = unit64(b3.z, b3.w);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        double* irp = (h == 0) ? &ir[k1] : &ir[k2];
+        double& irp = (h == 0) ? p.i : q.i;
         if (uRel[h] <= C.prelax) {
-            const double preEr = *irp;
+            const double preEr = irp;
             const double postEr = dm(da(preErt, preEr), ds(1.0, pow(rRel[h], C.expLB)));
-            *irp = postEr;
+            irp = postEr;
             preErt = ds(da(preErt, preEr), postEr);
         }
     }
     const double postVr = sqrt(dd(dm(2.0, preErt), 0.5));
-    const double vc0 = dm(0.5, da(v1x, v2x)), vc1 = dm(0.5, da(v1y, v2y)), vc2 = dm(0.5, da(v1z, v2z));
+    const double vc0 = dm(0.5, da(p.x, q.x)), vc1 = dm(0.5, da(p.y, q.y)), vc2 = dm(0.5, da(p.z, q.z));
     const double cosChi = ds(dm(2.0, pow(rChi, C.invAlpha)), 1.0);
     const double sinChi = sqrt(ds(1.0, dm(cosChi, cosChi)));
     const double ang = dm(6.283185307179586, th);   // 2 pi th
@@ -966,36 +968,33 @@ __device__ __forceinline__ void pair_execute_fp64(double* vx, double* vy, double
         r2 = dm(scale, da(dm(cosChi, vr1), dd(dm(sinChi, ds(dm(dm(cr, vr2), cth), dm(dm(vr0, vr1), sth))), vrpc)));
         r3 = dm(scale, ds(dm(cosChi, vr2), dd(dm(sinChi, da(dm(dm(cr, vr1), cth), dm(dm(vr0, vr2), sth))), vrpc)));
     }
-    vx[k1] = da(vc0, dm(0.5, r1)); vy[k1] = da(vc1, dm(0.5, r2)); vz[k1] = da(vc2, dm(0.5, r3));
-    vx[k2] = ds(vc0, dm(0.5, r1)); vy[k2] = ds(vc1, dm(0.5, r2)); vz[k2] = ds(vc2, dm(0.5, r3));
+    p.x = da(vc0, dm(0.5, r1)); p.y = da(vc1, dm(0.5, r2)); p.z = da(vc2, dm(0.5, r3));
+    q.x = ds(vc0, dm(0.5, r1)); q.y = ds(vc1, dm(0.5, r2)); q.z = ds(vc2, dm(0.5, r3));
 }
 
-__device__ __forceinline__ void pair_execute_fp32(float* vx, float* vy, float* vz, float* ir, int k1, int k2,
-                                                  const PairDraw& d, uint32_t w3, const DevConsts& C)
+__device__ __forceinline__ void pair_execute_fp32(PState<float>& p, PState<float>& q, const U4& b1, uint32_t w3,
+                                                  const DevConsts& C)
 {
-    const float v1x = vx[k1], v1y = vy[k1], v1z = vz[k1];
-    const float v2x = vx[k2], v2y = vy[k2], v2z = vz[k2];
-    const float vr0 = v1x - v2x, vr1 = v1y - v2y, vr2 = v1z - v2z;
+    const float vr0 = p.x - q.x, vr1 = p.y - q.y, vr2 = p.z - q.z;
     const float cr2 = vr0 * vr0 + vr1 * vr1 + vr2 * vr2;
     const float cr = psqrt(cr2);
     float preErt = 0.25f * cr2;
-    const U4 b1 = d.block(1, C);
     const float uRel[2] = {unit32(w3), unit32(b1.x)};
     const float rChi = unit32(b1.y), th = unit32(b1.z);
     const float expLB = (float)C.expLB;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        float* irp = (h == 0) ? &ir[k1] : &ir[k2];
+        float& irp = (h == 0) ? p.i : q.i;
         if (uRel[h] <= C.prelaxF) {
             const float r = fminf(uRel[h] * C.invPrelaxF, 1.0f);
-            const float preEr = *irp;
+            const float preEr = irp;
             const float postEr = (preErt + preEr) * (1.0f - exp2f(expLB * __log2f(r)));
-            *irp = postEr;
+            irp = postEr;
             preErt = preErt + preEr - postEr;
         }
     }
     const float postVr = 2.0f * psqrt(preErt);
-    const float vc0 = 0.5f * (v1x + v2x), vc1 = 0.5f * (v1y + v2y), vc2 = 0.5f * (v1z + v2z);
+    const float vc0 = 0.5f * (p.x + q.x), vc1 = 0.5f * (p.y + q.y), vc2 = 0.5f * (p.z + q.z);
     const float cosChi =
         (C.alpha == 1.0) ? 2.0f * rChi - 1.0f : 2.0f * exp2f((float)C.invAlpha * __log2f(rChi)) - 1.0f;
     const float sinChi = psqrt(1.0f - cosChi * cosChi);
@@ -1015,18 +1014,32 @@ __device__ __forceinline__ void pair_execute_fp32(float* vx, float* vy, float* v
         r2 = scale * (cosChi * vr1 + __fdividef(sinChi * (cr * vr2 * cth - vr0 * vr1 * sth), vrpc));
         r3 = scale * (cosChi * vr2 - __fdividef(sinChi * (cr * vr1 * cth + vr0 * vr2 * sth), vrpc));
     }
-    vx[k1] = vc0 + 0.5f * r1; vy[k1] = vc1 + 0.5f * r2; vz[k1] = vc2 + 0.5f * r3;
-    vx[k2] = vc0 - 0.5f * r1; vy[k2] = vc1 - 0.5f * r2; vz[k2] = vc2 - 0.5f * r3;
+    p.x = vc0 + 0.5f * r1; p.y = vc1 + 0.5f * r2; p.z = vc2 + 0.5f * r3;
+    q.x = vc0 - 0.5f * r1; q.y = vc1 - 0.5f * r2; q.z = vc2 - 0.5f * r3;
 }
 
+// One candidate pair (j of cell c) on the two particles' states: tested and,
+// when accepted, carried out. The draws of the second half do not depend on
+// the test, so in FP32 they are made beside it (the lanes of a warp that
+// reject would wait for those that accept in any case). Returns whether the
+// pair was accepted; crmLocal takes the relative speed if it is larger.
 template <typename Real>
-__device__ __forceinline__ void pair_execute(Real* vx, Real* vy, Real* vz, Real* ir, int stride, int k1, int k2,
-                                             int c, int istep, int j, uint32_t w3, const DevConsts& C)
+__device__ __forceinline__ bool pair_collide(PState<Real>& p, PState<Real>& q, int c, int istep, int j, uint32_t w2,
+                                             uint32_t w3, const DevConsts& C, double consCrm, Real crm0, bool splitSum,
+                                             Real& crmLocal)
 {
     PairDraw d;
     d.c = (uint32_t)c; d.istep = (uint32_t)istep; d.purpose = kPurposeCollide | ((uint32_t)j << 4);
-    if constexpr (sizeof(Real) == 8) pair_execute_fp64(vx, vy, vz, ir, k1 * stride, k2 * stride, d, C);
-    else pair_execute_fp32(vx, vy, vz, ir, k1 * stride, k2 * stride, d, w3, C);
+    U4 b1;
+    if constexpr (sizeof(Real) == 4) b1 = d.block(1, C);
+    Real cr;
+    const bool acc = pair_accept<Real>(p, q, w2, w3, C, consCrm, crm0, splitSum, cr);
+    if (cr > crmLocal) crmLocal = cr;
+    if (acc) {
+        if constexpr (sizeof(Real) == 8) pair_execute_fp64(p, q, d, C);
+        else pair_execute_fp32(p, q, b1, w3, C);
+    }
+    return acc;
 }
 
 // Candidate pair count of a cell from the majorant, with the carried
@@ -1050,70 +1063,51 @@ __device__ __forceinline__ int pair_count(const StepArgs<Real>& a, int c, int n,
     return npairs;
 }
 
-// The pair count and the majorant term of cell c as the classify pass
-// computed them (pair_count), with the cell's crmax.
-template <typename Real>
-__device__ __forceinline__ int pair_fetch(const StepArgs<Real>& a, int c, double& consCrm, double& crm0)
-{
-    consCrm = a.cellCons[c];
-    crm0 = a.crmax[c];
-    return a.cellPairs[c];
-}
-
 // NTC collisions of one small cell by one thread: the candidate pairs one
-// after another, particle k at v[k * stride].
+// after another, component q of particle k at v[q][k * stride].
 template <typename Real>
-__device__ void collide_cell_serial(Real* vx, Real* vy, Real* vz, Real* ir, int stride, int n, int c,
-                                    const StepArgs<Real>& a, int istep, uint32_t& pairsOut, uint32_t& collOut)
+__device__ void collide_cell_serial(Real* const (&v)[4], int stride, int n, int c, const StepArgs<Real>& a, int istep,
+                                    uint32_t& collOut)
 {
-    if (n <= 1) return;
-    double consCrm, crm0;
-    const int npairs = pair_fetch(a, c, consCrm, crm0);
-    pairsOut += (uint32_t)npairs;
+    const int npairs = a.cellPairs[c];
+    const double consCrm = a.cellCons[c], crm0 = a.crmax[c];
     if (!(consCrm > 0.0) || npairs <= 0) return;
     Real crmLocal = (Real)0;
     const Real crm0r = (Real)crm0;
+    auto load = [&](int k) { return PState<Real>{v[0][k * stride], v[1][k * stride], v[2][k * stride], v[3][k * stride]}; };
+    auto store = [&](int k, const PState<Real>& p) {
+        v[0][k * stride] = p.x; v[1][k * stride] = p.y; v[2][k * stride] = p.z; v[3][k * stride] = p.i;
+    };
     for (int j = 0; j < npairs; ++j) {
         int k1, k2;
         const PairDraw d = pair_draw(c, istep, j, n, a.C, k1, k2);
-        if (pair_accept<Real>(vx, vy, vz, stride, k1, k2, d.b0.z, d.b0.w, a.C, consCrm, crm0r, crmLocal)) {
-            pair_execute<Real>(vx, vy, vz, ir, stride, k1, k2, c, istep, j, d.b0.w, a.C);
+        PState<Real> p = load(k1), q = load(k2);
+        if (pair_collide<Real>(p, q, c, istep, j, d.b0.z, d.b0.w, a.C, consCrm, crm0r, true, crmLocal)) {
+            store(k1, p);
+            store(k2, q);
             ++collOut;
         }
     }
     if ((double)crmLocal > crm0) a.crmax[c] = (double)crmLocal;
 }
 
-// NTC collisions of one cell by one warp (collisionDSMC,
-// src/ProcessDSMC.cpp:2631-2665): the pair count from the majorant with the
-// carried remainder, then candidate pairs j = 0, 1, ... each drawn from a
-// Philox stream keyed by (cell, step, j).
-//
-// The pairs run as a sliding window: every lane holds one pending pair and
-// claims both its particles with the pair index (atomicMin); a pair whose
-// index is the lowest claim on both particles goes, and its lane takes the
-// next unassigned pair. Pairs are handed out in increasing order, so a pair
-// goes only after every lower pair that shares a particle with it, and the
-// result equals running the pairs one after another. The lowest pending
-// pair always goes, so the loop ends after at most npairs rounds.
-// claim holds n ints (shared memory, or the output buffer's cell-id slots
-// of the cell for large cells; the caller restores those).
+// NTC collisions of one cell by one warp, in place in the particle buffer,
+// for cells beyond every shared-memory arena. The pairs run as a sliding
+// window: every lane holds one pending pair and claims both its particles
+// with the pair index (atomicMin); a pair whose index is the lowest claim on
+// both particles goes, and its lane takes the next unassigned pair. Pairs are
+// handed out in increasing order, so a pair goes only after every lower pair
+// that shares a particle with it, and the result equals running the pairs one
+// after another. The lowest pending pair always goes, so the loop ends after
+// at most npairs rounds. The claims sit in the cell-id slots of the cell and
+// are replaced by the cell id at the end.
 template <typename Real>
-__device__ void collide_cell(Real* vx, Real* vy, Real* vz, Real* ir, int* claim, int n, int c,
-                             const StepArgs<Real>& a, int istep, uint32_t& pairsOut, uint32_t& collOut)
+__device__ void collide_cell_in_place(const PBuf<Real>& buf, int s0, int n, int c, int npairs, double consCrm,
+                                      double crm0, const StepArgs<Real>& a, int istep, uint32_t& collOut)
 {
     const int lane = threadIdx.x & 31;
-    if (n <= 1) return;
-    double consCrm = 0.0, crm0 = 0.0;
-    int npairs = 0;
-    if (lane == 0) {
-        npairs = pair_fetch(a, c, consCrm, crm0);
-        pairsOut += (uint32_t)npairs;
-    }
-    npairs = __shfl_sync(kFull, npairs, 0);
-    consCrm = __shfl_sync(kFull, consCrm, 0);
-    crm0 = __shfl_sync(kFull, crm0, 0);
-    if (!(consCrm > 0.0) || npairs <= 0) return;
+    int* claim = buf.cell + s0;
+    Real* const v[4] = {buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0};
     for (int k = lane; k < n; k += 32) claim[k] = INT_MAX;
     __syncwarp();
     Real crmLocal = (Real)0;
@@ -1142,8 +1136,10 @@ __device__ void collide_cell(Real* vx, Real* vy, Real* vz, Real* ir, int* claim,
         const bool go = j >= 0 && claim[k1] == j && claim[k2] == j;
         __syncwarp();
         if (go) {
-            if (pair_accept<Real>(vx, vy, vz, 1, k1, k2, d.b0.z, d.b0.w, a.C, consCrm, crm0r, crmLocal)) {
-                pair_execute<Real>(vx, vy, vz, ir, 1, k1, k2, c, istep, j, d.b0.w, a.C);
+            PState<Real> p{v[0][k1], v[1][k1], v[2][k1], v[3][k1]}, q{v[0][k2], v[1][k2], v[2][k2], v[3][k2]};
+            if (pair_collide<Real>(p, q, c, istep, j, d.b0.z, d.b0.w, a.C, consCrm, crm0r, true, crmLocal)) {
+                v[0][k1] = p.x; v[1][k1] = p.y; v[2][k1] = p.z; v[3][k1] = p.i;
+                v[0][k2] = q.x; v[1][k2] = q.y; v[2][k2] = q.z; v[3][k2] = q.i;
                 ++collOut;
             }
             claim[k1] = INT_MAX;
@@ -1159,68 +1155,156 @@ __device__ void collide_cell(Real* vx, Real* vy, Real* vz, Real* ir, int* claim,
         m = y > m ? y : m;
     }
     if (lane == 0 && (double)m > crm0) a.crmax[c] = (double)m;
+    for (int k = lane; k < n; k += 32) claim[k] = c;
+    __syncwarp();
 }
 
 // The collision pass over the sorted buffer (collisionDSMC,
-// src/ProcessDSMC.cpp:2621-2665). Cells are classified first
-// (classify_kernel) and handed out dynamically, largest first:
-// - huge cells (more than kArena particles): one at a time by a whole warp
-//   (collide_cell), in place in the buffer;
-// - large cells: two at a time per warp (collide_two_channels), staged in
-//   shared memory;
+// src/ProcessDSMC.cpp:2621-2665). Cells are classed first (classify_kernel):
 // - small cells (at most kSmallMax particles): 32 at a time per warp, lane
 //   l owning one cell and running its pairs alone, with the particles'
 //   velocities and internal energies in shared memory at slot k * 32 + l
-//   (lane l's slots sit in bank l, so the lanes never conflict).
-// A cell's result depends on nothing but the cell, so neither the warp that
-// takes it nor the order matters.
-constexpr int kCellWarps = 2;
+//   (lane l's slots sit in bank l, so the lanes never conflict);
+// - large cells: two at a time per warp, staged in shared memory
+//   (collide_kernel);
+// - big cells (more particles than a warp's arena, or more pairs than
+//   kBigPairs) and giants (more pairs than kGiantPairs, handed out first):
+//   one at a time by a block of 512 threads (collide_big_kernel), beside the
+//   other kernel on the side stream.
+// A cell's result depends on nothing but the cell, so neither the warp or
+// block that takes it nor the order matters.
+//
+// What bounds it: a cell's pairs depend on each other through its particles,
+// so a cell is a chain of rounds, and the pass is as long as the longest
+// chain. With every cell run by one warp, 32 pairs a round at most, the few
+// compressed cells of a capsule (2,000 particles, 30,000-60,000 pairs) were
+// the whole pass. A block runs up to 512 pairs a round (n / 4 (1 - e^(-2048 / n))
+// of them go), in a tenth of the rounds.
+constexpr int kCellWarps = 2;                 // warps per block of collide_kernel
 constexpr int kSmallMax = 16;
 constexpr int kArena = 512;                   // staged particles per warp
-constexpr int kSmallSlots = 32 * kSmallMax;
-static_assert(kSmallSlots <= kArena, "small-cell slots must fit in the arena");
+static_assert(32 * kSmallMax <= kArena, "small-cell slots must fit in the arena");
+constexpr int kBigThreads = 512;
+constexpr int kBigArena = 4096;               // staged particles per block of collide_big_kernel
+constexpr int kBigPairs = 1024;
+constexpr int kGiantPairs = 8192;
 
-// per-warp shared memory: Real arena[4][kArena]; int claim[kArena]; int4 queue[64]
+// shared memory of `slots` staged particles: their states and claims
 template <typename Real>
-__host__ __device__ constexpr size_t warp_smem_bytes()
+__host__ __device__ constexpr size_t arena_bytes(int slots)
 {
-    return (size_t)kArena * (4 * sizeof(Real) + sizeof(int)) + 64 * sizeof(int4);
-}
-template <typename Real>
-__host__ __device__ constexpr size_t cell_smem_bytes()
-{
-    return (size_t)kCellWarps * warp_smem_bytes<Real>();
+    return (size_t)slots * (4 * sizeof(Real) + sizeof(int));
 }
 
-// cellWork: [0] huge count, [1] large count, [2] small count,
-//           [3] next huge/large item, [4] next small item
-// cellList: huge cells from the front of [0, ncell), large cells from its
-//           back, small cells from the front of [ncell, 2 ncell)
+// particle states in shared memory, 16 bytes a load
 template <typename Real>
-__global__ void classify_kernel(StepArgs<Real> a, int stageMax)
+struct Arena;
+template <>
+struct Arena<float> {
+    float4* v;
+    int* claim;
+    __device__ __forceinline__ Arena(unsigned char* p, int slots)
+        : v(reinterpret_cast<float4*>(p)), claim(reinterpret_cast<int*>(v + slots))
+    {
+    }
+    __device__ __forceinline__ PState<float> get(int k) const
+    {
+        const float4 t = v[k];
+        return {t.x, t.y, t.z, t.w};
+    }
+    __device__ __forceinline__ void put(int k, const PState<float>& p) const { v[k] = make_float4(p.x, p.y, p.z, p.i); }
+};
+template <>
+struct Arena<double> {
+    double2 *lo, *hi;
+    int* claim;
+    __device__ __forceinline__ Arena(unsigned char* p, int slots)
+        : lo(reinterpret_cast<double2*>(p)), hi(lo + slots), claim(reinterpret_cast<int*>(hi + slots))
+    {
+    }
+    __device__ __forceinline__ PState<double> get(int k) const
+    {
+        const double2 s = lo[k], t = hi[k];
+        return {s.x, s.y, t.x, t.y};
+    }
+    __device__ __forceinline__ void put(int k, const PState<double>& p) const
+    {
+        lo[k] = make_double2(p.x, p.y);
+        hi[k] = make_double2(p.z, p.i);
+    }
+};
+
+// Stage a cell (n particles from s0) at arena slots base.., by T threads of
+// which this is thread t: the loads of four particles a thread are issued
+// before their stores. unstage writes it back.
+template <typename Real>
+__device__ __forceinline__ void stage_cell(const PBuf<Real>& buf, const Arena<Real>& A, int s0, int n, int base, int t,
+                                           int T)
+{
+    for (int k0 = t; k0 < n; k0 += 4 * T) {
+        PState<Real> p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + u * T;
+            if (k < n) p[u] = {buf.v[0][s0 + k], buf.v[1][s0 + k], buf.v[2][s0 + k], buf.ir[s0 + k]};
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + u * T;
+            if (k < n) {
+                A.put(base + k, p[u]);
+                A.claim[base + k] = INT_MAX;
+            }
+        }
+    }
+}
+template <typename Real>
+__device__ __forceinline__ void unstage_cell(const PBuf<Real>& buf, const Arena<Real>& A, int s0, int n, int base, int t,
+                                             int T)
+{
+    for (int k = t; k < n; k += T) {
+        const PState<Real> p = A.get(base + k);
+        buf.v[0][s0 + k] = p.x; buf.v[1][s0 + k] = p.y; buf.v[2][s0 + k] = p.z;
+        buf.ir[s0 + k] = p.i;
+    }
+}
+
+// cellWork: [0] large count, [1] small count, [2] big count, [3] giant count,
+//           [4] next large item, [5] next small item, [6] next giant or big
+// cellList: small cells from the front of [0, ncell), big cells from its
+//           back, giants from the front of [ncell, 2 ncell)
+// cellItem: large cells
+template <typename Real>
+__global__ void classify_kernel(StepArgs<Real> a)
 {
     const int lane = threadIdx.x & 31;
     const int* start = a.startA;
     const int ncell = a.M.ncell;
-    int* list = a.cellList;
     int* work = a.cellWork;
+    uint32_t pairs = 0, over = 0;
     for (int base = blockIdx.x * blockDim.x; base < ncell; base += gridDim.x * blockDim.x) {
         const int c = base + threadIdx.x;
         const int s0 = c < ncell ? start[c] : 0;
         const int n = c < ncell ? start[c + 1] - s0 : -1;
-        // the cell's candidate pair count, one thread per cell (the
-        // collision kernels read it back with pair_fetch, or from the
-        // cell's item record)
+        // the cell's candidate pair count, one thread per cell
         int np = 0;
         double consCrm = 0.0, crm0 = 0.0;
         if (n > 1) {
             np = pair_count(a, c, n, consCrm, crm0);
             a.cellPairs[c] = np;
             a.cellCons[c] = consCrm;
+            pairs += (uint32_t)np;
         }
-        const int cls = n < 0 ? -1 : (n > stageMax ? 0 : (n > kSmallMax ? 1 : 2));
+        if (n > 512) ++over;
+        // nothing collides in a cell without pairs: it goes on no list
+        int cls = -1;
+        if (n > 1 && np > 0 && consCrm > 0.0) {
+            if (n <= kSmallMax) cls = 1;
+            else if (np > kGiantPairs) cls = 3;
+            else cls = n > kArena || np > kBigPairs ? 2 : 0;
+        }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 4; ++k) {
             const unsigned m = __ballot_sync(kFull, cls == k);
             if (!m) continue;
             const int leader = __ffs(m) - 1;
@@ -1229,302 +1313,325 @@ __global__ void classify_kernel(StepArgs<Real> a, int stageMax)
             b = __shfl_sync(kFull, b, leader);
             if (cls == k) {
                 const int pos = b + __popc(m & ((1u << lane) - 1u));
-                if (k == 2) {
-                    list[ncell + pos] = c;
+                if (k == 0) {
+                    a.cellItem[pos] = make_int4(c, s0, n, np);
+                    a.cellItemC[pos] = make_double2(consCrm, crm0);
                 } else {
-                    const int slot = k == 0 ? pos : ncell - 1 - pos;
-                    list[slot] = c;
-                    a.cellItem[slot] = make_int4(c, s0, n, np);
-                    a.cellItemC[slot] = make_double2(consCrm, crm0);
+                    a.cellList[k == 1 ? pos : k == 2 ? ncell - 1 - pos : ncell + pos] = c;
                 }
             }
         }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        pairs += __shfl_xor_sync(kFull, pairs, o);
+        over += __shfl_xor_sync(kFull, over, o);
+    }
+    if (lane == 0) {
+        if (pairs) atomicAdd(a.counters + C_PAIRS, (unsigned long long)pairs);
+        if (over) atomicAdd(a.counters + C_BIG_CELLS, (unsigned long long)over);
+    }
 }
 
-// copy a cell's velocities and internal energies between the buffer (at s0)
-// and v[comp][k * stride], whole warp. Into shared memory, the loads of up
-// to 128 particles are issued before their stores (one round trip to
-// memory for most cells instead of one per 32 particles).
+// copy a small cell's velocities and internal energies between the buffer
+// (at s0) and v[comp][k * 32], whole warp
 template <typename Real, bool kToBuffer>
-__device__ __forceinline__ void copy_cell(const PBuf<Real>& buf, int s0, int n, Real* const (&v)[4], int stride)
+__device__ __forceinline__ void copy_cell(const PBuf<Real>& buf, int s0, int n, Real* const (&v)[4])
 {
-    const int lane = threadIdx.x & 31;
-    Real* b[4] = {buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0};
-    if constexpr (kToBuffer) {
-        for (int k = lane; k < n; k += 32)
+    Real* const b[4] = {buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0};
+    const int k = threadIdx.x & 31;
+    if (k < n)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) b[q][k] = v[q][k * stride];
-    } else {
-        for (int k0 = lane; k0 < n; k0 += 128) {
-            Real t[4][4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int k = k0 + 32 * u;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) t[u][q] = k < n ? b[q][k] : (Real)0;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int k = k0 + 32 * u;
-                if (k < n)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) v[q][k * stride] = t[u][q];
-            }
+        for (int q = 0; q < 4; ++q) {
+            if constexpr (kToBuffer) b[q][k] = v[q][k * 32];
+            else v[q][k * 32] = b[q][k];
         }
+}
+
+// the largest of a warp's values
+template <typename Real>
+__device__ __forceinline__ Real warp_max(Real m)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const Real y = __shfl_xor_sync(kFull, m, o);
+        m = y > m ? y : m;
     }
+    return m;
 }
 
 // Collisions of staged large cells, two cells per warp at a time, both in
 // the warp's arena: channel 0's cell at slots [0, n0), channel 1's at
 // [kArena - n1, kArena); a cell that does not fit beside the other channel's
-// waits until that one is done. Each channel runs the sliding window of
-// collide_cell (one pending pair per lane, claims by pair index); the pairs
-// that go in a round are tested for acceptance by their own lanes, and the
-// accepted ones, from both channels, are queued in shared memory and carried
-// out by consecutive lanes, so the costly half of a collision runs once per
-// round with most lanes busy. A channel whose pairs are done writes its
-// cell back and takes the next. *item holds a cell item
-// already taken from the list, or -1.
+// waits until that one is done. The pairs run as a sliding window: every
+// lane holds one pending pair of either cell and claims its two particles
+// with the pair index (atomicMin); a pair whose index is the lowest claim on
+// both goes, tested and carried out by its lane, which then takes the next
+// pair not yet handed out: of channel 0 in the lower half of the warp, of
+// channel 1 in the upper, or of the other channel when its own has none
+// left. A cell's pairs are handed out in increasing order, so a pair goes
+// only after every lower pair that shares a particle with it, and the result
+// equals running the pairs one after another. The lowest pending pair of a
+// cell always goes, so the loop ends after at most the pairs' number of
+// rounds. A channel whose pairs are done writes its cell back and takes the
+// next.
+// Half a warp per cell, because of 32 pairs of one cell of 100-300 particles
+// some 13 to 20 go a round, and of 16 about 13; each phase then runs once a
+// round for both cells.
 template <typename Real>
-__device__ void collide_two_channels(const StepArgs<Real>& a, const PBuf<Real>& dst, const int* start, Real* arena,
-                                     int* sclaim, int4* queue, int nItems, int nHuge, int istep, int item,
-                                     uint32_t& pairs, uint32_t& colls)
+__device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf, const Arena<Real>& A, int nItems,
+                                  int istep, uint32_t& colls)
 {
     constexpr int N = kArena;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const int ncell = a.M.ncell;
     int cc[2] = {-1, -1}, cbase[2] = {0, 0}, cs0[2] = {0, 0}, cn[2] = {0, 0}, cnp[2] = {0, 0}, cnext[2] = {0, 0};
     double ccons[2] = {0.0, 0.0}, ccrm[2] = {0.0, 0.0};
     Real crmL[2] = {(Real)0, (Real)0};
-    int sj[2] = {-1, -1}, sk1[2] = {0, 0}, sk2[2] = {0, 0};
-    uint32_t sw2[2] = {0u, 0u}, sw3[2] = {0u, 0u};
-    int held = item;      // an item taken but not yet placed
+    int j = -1, ch = 0, k1 = 0, k2 = 0;   // this lane's pending pair
+    uint32_t w2 = 0u, w3 = 0u;
+    int held = -1;        // an item taken but not yet placed
     bool more = true;
     // the next item index, taken one item ahead (lane 0): the atomic's
     // round trip overlaps the rounds of the cells in work. Indices are
     // handed out in increasing order and the loop runs until it sees one
     // past the end, so an index taken ahead is always used.
     int ahead = 0;
-    if (lane == 0) ahead = atomicAdd(a.cellWork + 3, 1);
+    if (lane == 0) ahead = atomicAdd(a.cellWork + 4, 1);
     for (;;) {
 #pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            while (cc[ch] < 0 && (more || held >= 0)) {
+        for (int h = 0; h < 2; ++h) {
+            while (cc[h] < 0 && (more || held >= 0)) {
                 int it = held;
                 if (it < 0) {
                     it = __shfl_sync(kFull, ahead, 0);
-                    if (lane == 0 && it < nItems) ahead = atomicAdd(a.cellWork + 3, 1);
+                    if (lane == 0 && it < nItems) ahead = atomicAdd(a.cellWork + 4, 1);
                 }
                 held = -1;
                 if (it >= nItems) {
                     more = false;
                     break;
                 }
-                // the item's record (classify pass): one load instead of the
-                // list, the starts and the pair count one after another
-                const int slot = it < nHuge ? it : ncell - 1 - (it - nHuge);
-                const int4 rec = a.cellItem[slot];
-                const double2 rc = a.cellItemC[slot];
-                const int c = rec.x, s0 = rec.y, n = rec.z;
-                if (n > N) {   // never reached (huge items precede these): flag rather than overflow the arena
+                const int4 rec = a.cellItem[it];
+                const double2 rc = a.cellItemC[it];
+                const int n = rec.z;
+                if (n > N) {   // never reached (classify lists no such cell): flag rather than overflow the arena
                     if (lane == 0) atomicOr(a.errorWord, kErrStageCell);
                     continue;
                 }
-                if (n > N - (cc[ch ^ 1] >= 0 ? cn[ch ^ 1] : 0)) {   // wait for the other channel
+                if (n > N - (cc[h ^ 1] >= 0 ? cn[h ^ 1] : 0)) {   // wait for the other channel
                     held = it;
                     break;
                 }
-                const int np = n > 1 ? rec.w : 0;
-                const double consCrm = rc.x, crm0 = rc.y;
-                if (lane == 0) pairs += (uint32_t)np;
-                if (!(consCrm > 0.0) || np <= 0) continue;   // nothing changes: not staged
-                const int base = ch == 0 ? 0 : N - n;
-                Real* const v[4] = {arena + base, arena + N + base, arena + 2 * N + base, arena + 3 * N + base};
-                copy_cell<Real, false>(dst, s0, n, v, 1);
+                const int base = h == 0 ? 0 : N - n;
+                stage_cell(buf, A, rec.y, n, base, lane, 32);
+                cc[h] = rec.x; cbase[h] = base; cs0[h] = rec.y; cn[h] = n; cnp[h] = rec.w; cnext[h] = 0;
+                ccons[h] = rc.x; ccrm[h] = rc.y; crmL[h] = (Real)0;
                 __syncwarp();
-                for (int k = lane; k < n; k += 32) sclaim[base + k] = INT_MAX;
-                __syncwarp();
-                cc[ch] = c; cbase[ch] = base; cs0[ch] = s0; cn[ch] = n; cnp[ch] = np; cnext[ch] = 0;
-                ccons[ch] = consCrm; ccrm[ch] = crm0; crmL[ch] = (Real)0;
             }
         }
         if (cc[0] < 0 && cc[1] < 0) break;
         // hand out the next pairs to idle lanes
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            if (cc[ch] < 0) continue;
-            const unsigned idle = __ballot_sync(kFull, sj[ch] < 0);
-            if (sj[ch] < 0) {
-                const int jj = cnext[ch] + __popc(idle & below);
-                if (jj < cnp[ch]) {
-                    sj[ch] = jj;
-                    int k1, k2;
-                    const PairDraw d = pair_draw(cc[ch], istep, jj, cn[ch], a.C, k1, k2);
-                    sk1[ch] = cbase[ch] + k1;
-                    sk2[ch] = cbase[ch] + k2;
-                    sw2[ch] = d.b0.z;
-                    sw3[ch] = d.b0.w;
-                }
+        const bool left0 = cc[0] >= 0 && cnext[0] < cnp[0], left1 = cc[1] >= 0 && cnext[1] < cnp[1];
+        const int want = j >= 0 ? -1 : lane < 16 ? (left0 ? 0 : left1 ? 1 : -1) : (left1 ? 1 : left0 ? 0 : -1);
+        const unsigned m0 = __ballot_sync(kFull, want == 0), m1 = __ballot_sync(kFull, want == 1);
+        if (want >= 0) {
+            const int jj = (want ? cnext[1] : cnext[0]) + __popc((want ? m1 : m0) & below);
+            if (jj < (want ? cnp[1] : cnp[0])) {
+                j = jj;
+                ch = want;
+                const int base = want ? cbase[1] : cbase[0];
+                const PairDraw d = pair_draw(want ? cc[1] : cc[0], istep, jj, want ? cn[1] : cn[0], a.C, k1, k2);
+                k1 += base;
+                k2 += base;
+                w2 = d.b0.z;
+                w3 = d.b0.w;
             }
-            cnext[ch] = min(cnp[ch], cnext[ch] + __popc(idle));
         }
+        cnext[0] = min(cnp[0], cnext[0] + __popc(m0));
+        cnext[1] = min(cnp[1], cnext[1] + __popc(m1));
         // claim both particles with the pair index; the lowest claim goes
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch)
-            if (sj[ch] >= 0) {
-                atomicMin(&sclaim[sk1[ch]], sj[ch]);
-                atomicMin(&sclaim[sk2[ch]], sj[ch]);
-            }
-        __syncwarp();
-        bool go[2], acc[2];
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) go[ch] = sj[ch] >= 0 && sclaim[sk1[ch]] == sj[ch] && sclaim[sk2[ch]] == sj[ch];
-        __syncwarp();
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            acc[ch] = false;
-            if (go[ch])
-                acc[ch] = pair_accept<Real>(arena, arena + N, arena + 2 * N, 1, sk1[ch], sk2[ch], sw2[ch], sw3[ch], a.C,
-                                            ccons[ch], (Real)ccrm[ch], crmL[ch]);
+        if (j >= 0) {
+            atomicMin(&A.claim[k1], j);
+            atomicMin(&A.claim[k2], j);
         }
-        const unsigned m0 = __ballot_sync(kFull, acc[0]);
-        const unsigned m1 = __ballot_sync(kFull, acc[1]);
-        if (acc[0]) queue[__popc(m0 & below)] = make_int4(sk1[0] - cbase[0], sk2[0] - cbase[0], sj[0], (int)sw3[0]);
-        if (acc[1])
-            queue[__popc(m0) + __popc(m1 & below)] =
-                make_int4(sk1[1] - cbase[1], sk2[1] - cbase[1], sj[1] | (1 << 30), (int)sw3[1]);
         __syncwarp();
-        const int total = __popc(m0) + __popc(m1);
-        for (int e = lane; e < total; e += 32) {
-            const int4 q = queue[e];
-            const int ch = q.z >> 30;
-            const int base = ch ? cbase[1] : cbase[0];
-            Real* b = arena + base;
-            pair_execute<Real>(b, b + N, b + 2 * N, b + 3 * N, 1, q.x, q.y, ch ? cc[1] : cc[0], istep,
-                               q.z & 0x3fffffff, (uint32_t)q.w, a.C);
-        }
-        if (lane == 0) colls += (uint32_t)total;
+        const bool go = j >= 0 && A.claim[k1] == j && A.claim[k2] == j;
         __syncwarp();
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch)
-            if (go[ch]) {
-                sclaim[sk1[ch]] = INT_MAX;
-                sclaim[sk2[ch]] = INT_MAX;
-                sj[ch] = -1;
+        if (go) {
+            PState<Real> p = A.get(k1), q = A.get(k2);
+            Real& crm = ch ? crmL[1] : crmL[0];
+            if (pair_collide<Real>(p, q, ch ? cc[1] : cc[0], istep, j, w2, w3, a.C, ch ? ccons[1] : ccons[0],
+                                   (Real)(ch ? ccrm[1] : ccrm[0]), false, crm)) {
+                A.put(k1, p);
+                A.put(k2, q);
+                ++colls;
             }
+            A.claim[k1] = INT_MAX;
+            A.claim[k2] = INT_MAX;
+            j = -1;
+        }
         __syncwarp();
         // a channel whose pairs are all done finishes its cell
 #pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-            if (cc[ch] < 0) continue;
-            if (__ballot_sync(kFull, sj[ch] >= 0) != 0u || cnext[ch] < cnp[ch]) continue;
-            Real m = crmL[ch];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const Real y = __shfl_xor_sync(kFull, m, o);
-                m = y > m ? y : m;
-            }
-            if (lane == 0 && (double)m > ccrm[ch]) a.crmax[cc[ch]] = (double)m;
-            const int base = cbase[ch];
-            Real* const v[4] = {arena + base, arena + N + base, arena + 2 * N + base, arena + 3 * N + base};
-            copy_cell<Real, true>(dst, cs0[ch], cn[ch], v, 1);
+        for (int h = 0; h < 2; ++h) {
+            if (cc[h] < 0 || cnext[h] < cnp[h] || __ballot_sync(kFull, j >= 0 && ch == h) != 0u) continue;
+            const Real m = warp_max(crmL[h]);
+            if (lane == 0 && (double)m > ccrm[h]) a.crmax[cc[h]] = (double)m;
+            unstage_cell(buf, A, cs0[h], cn[h], cbase[h], lane, 32);
             __syncwarp();
-            cc[ch] = -1;
+            cc[h] = -1;
         }
     }
 }
 
-// Nine resident blocks (18 warps) per SM: the arena (22.5 KB per block plus
-// the 1 KB the runtime reserves) fits nine in 228 KB; the bound caps the
-// registers to match (113 per thread).
+// Ten resident blocks (20 warps) per SM in FP32, six in FP64: the arenas
+// (20 and 36 KB per block plus the 1 KB the runtime reserves) fill the 228 KB.
 template <typename Real>
-__global__ void __launch_bounds__(kCellWarps * 32, 9) collide_kernel(StepArgs<Real> a)
+__global__ void __launch_bounds__(kCellWarps * 32, sizeof(Real) == 4 ? 10 : 6) collide_kernel(StepArgs<Real> a)
 {
     extern __shared__ __align__(16) unsigned char cellSmem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    unsigned char* wsm = cellSmem + (size_t)wib * warp_smem_bytes<Real>();
-    Real* sv = reinterpret_cast<Real*>(wsm);
-    int* sclaim = reinterpret_cast<int*>(wsm + (size_t)4 * kArena * sizeof(Real));
-    int4* queue = reinterpret_cast<int4*>(wsm + (size_t)kArena * (4 * sizeof(Real) + sizeof(int)));
-    Real* const stage[4] = {sv, sv + kSmallSlots, sv + 2 * kSmallSlots, sv + 3 * kSmallSlots};
+    unsigned char* const wsm = cellSmem + (size_t)wib * arena_bytes<Real>(kArena);
     const int istep = a.ctl->istep;
     const PBuf<Real> buf = a.A;
-    const int* start = a.startA;
-    const int ncell = a.M.ncell;
-    const int nHuge = a.cellWork[0], nLarge = a.cellWork[1], nSmall = a.cellWork[2];
-    uint32_t pairs = 0, colls = 0, big = 0;
+    uint32_t colls = 0;
 
-    // ---- huge cells, one at a time by the whole warp, in place
-    int item = -1;
-    for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(a.cellWork + 3, 1);
-        it = __shfl_sync(kFull, it, 0);
-        if (it >= nHuge + nLarge) break;
-        if (it >= nHuge) {   // a large cell: the two-channel loop takes it
-            item = it;
-            break;
-        }
-        const int c = a.cellList[it];
-        const int s0 = start[c];
-        const int n = start[c + 1] - s0;
-        if (lane == 0) ++big;
-        collide_cell<Real>(buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0, buf.cell + s0, n, c, a, istep,
-                           pairs, colls);
-        __syncwarp();
-        for (int k = lane; k < n; k += 32) buf.cell[s0 + k] = c;   // the claims used the cell ids
-        __syncwarp();
-    }
-
-    // ---- large cells, two at a time
-    if (item >= 0)
-        collide_two_channels<Real>(a, buf, start, sv, sclaim, queue, nHuge + nLarge, nHuge, istep, item, pairs, colls);
+    const int nLarge = a.cellWork[0], nSmall = a.cellWork[1];
+    if (nLarge > 0) collide_two_cells<Real>(a, buf, Arena<Real>(wsm, kArena), nLarge, istep, colls);
 
     // ---- small cells, 32 per warp, one lane each
-    for (;;) {
+    constexpr int kSmallSlots = 32 * kSmallMax;
+    Real* const sv = reinterpret_cast<Real*>(wsm);
+    Real* const stage[4] = {sv, sv + kSmallSlots, sv + 2 * kSmallSlots, sv + 3 * kSmallSlots};
+    const int* start = a.startA;
+    while (nSmall > 0) {
         int g = 0;
-        if (lane == 0) g = atomicAdd(a.cellWork + 4, 32);
+        if (lane == 0) g = atomicAdd(a.cellWork + 5, 32);
         g = __shfl_sync(kFull, g, 0);
         if (g >= nSmall) break;
         const bool mine = g + lane < nSmall;
-        const int myc = mine ? a.cellList[ncell + g + lane] : 0;
+        const int myc = mine ? a.cellList[g + lane] : 0;
         const int ms0 = mine ? start[myc] : 0;
         const int mn = mine ? start[myc + 1] - ms0 : 0;
-        const unsigned mask = __ballot_sync(kFull, mine && mn > 1);
-        for (unsigned m = mask; m; m &= m - 1) {
-            const int l = __ffs(m) - 1;
+        const int many = min(32, nSmall - g);
+        for (int l = 0; l < many; ++l) {
             Real* const to[4] = {stage[0] + l, stage[1] + l, stage[2] + l, stage[3] + l};
-            copy_cell<Real, false>(buf, __shfl_sync(kFull, ms0, l), __shfl_sync(kFull, mn, l), to, 32);
+            copy_cell<Real, false>(buf, __shfl_sync(kFull, ms0, l), __shfl_sync(kFull, mn, l), to);
         }
         __syncwarp();
-        if ((mask >> lane) & 1u)
-            collide_cell_serial<Real>(stage[0] + lane, stage[1] + lane, stage[2] + lane, stage[3] + lane, 32, mn, myc,
-                                      a, istep, pairs, colls);
+        if (mine) {
+            Real* const v[4] = {stage[0] + lane, stage[1] + lane, stage[2] + lane, stage[3] + lane};
+            collide_cell_serial<Real>(v, 32, mn, myc, a, istep, colls);
+        }
         __syncwarp();
-        for (unsigned m = mask; m; m &= m - 1) {
-            const int l = __ffs(m) - 1;
+        for (int l = 0; l < many; ++l) {
             Real* const from[4] = {stage[0] + l, stage[1] + l, stage[2] + l, stage[3] + l};
-            copy_cell<Real, true>(buf, __shfl_sync(kFull, ms0, l), __shfl_sync(kFull, mn, l), from, 32);
+            copy_cell<Real, true>(buf, __shfl_sync(kFull, ms0, l), __shfl_sync(kFull, mn, l), from);
         }
         __syncwarp();
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        pairs += __shfl_xor_sync(kFull, pairs, o);
-        colls += __shfl_xor_sync(kFull, colls, o);
-        big += __shfl_xor_sync(kFull, big, o);
-    }
-    if (lane == 0) {
-        if (pairs) atomicAdd(a.counters + C_PAIRS, (unsigned long long)pairs);
-        if (colls) atomicAdd(a.counters + C_COLLISIONS, (unsigned long long)colls);
-        if (big) atomicAdd(a.counters + C_BIG_CELLS, (unsigned long long)big);
-    }
+    for (int o = 16; o > 0; o >>= 1) colls += __shfl_xor_sync(kFull, colls, o);
+    if (lane == 0 && colls) atomicAdd(a.counters + C_COLLISIONS, (unsigned long long)colls);
 }
 
-// resident blocks per SM of each cell-kernel variant, set by prepare_kernels
+// Big cells, one at a time by the whole block, giants first: the sliding
+// window of collide_two_cells over 512 threads. The idle threads of a warp
+// take their pairs together from a counter; which of them gets which pair
+// does not matter, only that every pair below a claimed one is claimed or
+// done, and the barrier before the claims are read sees to that.
+template <typename Real>
+__global__ void __launch_bounds__(kBigThreads, 1) collide_big_kernel(StepArgs<Real> a)
+{
+    extern __shared__ __align__(16) unsigned char cellSmem[];
+    __shared__ int sItem, sNext;
+    __shared__ unsigned long long sCrm;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const Arena<Real> A(cellSmem, kBigArena);
+    const int istep = a.ctl->istep, ncell = a.M.ncell;
+    const int nBig = a.cellWork[2], nGiant = a.cellWork[3];
+    const PBuf<Real> buf = a.A;
+    uint32_t colls = 0;
+    if (nBig + nGiant > 0)
+        for (;;) {
+            __syncthreads();   // the last cell's values have been read
+            if (tid == 0) {
+                sItem = atomicAdd(a.cellWork + 6, 1);
+                sNext = 0;
+                sCrm = 0ull;
+            }
+            __syncthreads();
+            const int it = sItem;
+            if (it >= nBig + nGiant) break;
+            const int c = a.cellList[it < nGiant ? ncell + it : ncell - 1 - (it - nGiant)];
+            const int s0 = a.startA[c], n = a.startA[c + 1] - s0, np = a.cellPairs[c];
+            const double consCrm = a.cellCons[c], crm0 = a.crmax[c];
+            if (n > kBigArena) {
+                if (tid < 32) collide_cell_in_place<Real>(buf, s0, n, c, np, consCrm, crm0, a, istep, colls);
+                continue;
+            }
+            stage_cell(buf, A, s0, n, 0, tid, kBigThreads);
+            __syncthreads();
+            const Real crm0r = (Real)crm0;
+            Real crmLocal = (Real)0;
+            int j = -1, k1 = 0, k2 = 0;
+            uint32_t w2 = 0u, w3 = 0u;
+            bool left = true;   // pairs may be left to hand out
+            for (;;) {
+                if (left) {     // the same in every lane of a warp
+                    const unsigned idle = __ballot_sync(kFull, j < 0);
+                    if (idle) {
+                        int first = 0;
+                        if (lane == 0) first = atomicAdd(&sNext, __popc(idle));
+                        first = __shfl_sync(kFull, first, 0);
+                        const int jj = first + __popc(idle & below);
+                        if (j < 0 && jj < np) {
+                            j = jj;
+                            const PairDraw d = pair_draw(c, istep, j, n, a.C, k1, k2);
+                            w2 = d.b0.z;
+                            w3 = d.b0.w;
+                        }
+                        left = first < np;
+                    }
+                }
+                if (j >= 0) {
+                    atomicMin(&A.claim[k1], j);
+                    atomicMin(&A.claim[k2], j);
+                }
+                __syncthreads();
+                const bool go = j >= 0 && A.claim[k1] == j && A.claim[k2] == j;
+                __syncthreads();
+                if (go) {
+                    PState<Real> p = A.get(k1), q = A.get(k2);
+                    if (pair_collide<Real>(p, q, c, istep, j, w2, w3, a.C, consCrm, crm0r, n > kArena,
+                                           crmLocal)) {
+                        A.put(k1, p);
+                        A.put(k2, q);
+                        ++colls;
+                    }
+                    A.claim[k1] = INT_MAX;
+                    A.claim[k2] = INT_MAX;
+                    j = -1;
+                }
+                if (!__syncthreads_or(left || j >= 0)) break;
+            }
+            // the largest relative speed tested (a double's order is that of
+            // its bits when positive)
+            const Real m = warp_max(crmLocal);
+            if (lane == 0 && (double)m > crm0) atomicMax(&sCrm, (unsigned long long)__double_as_longlong((double)m));
+            unstage_cell(buf, A, s0, n, 0, tid, kBigThreads);
+            __syncthreads();
+            if (tid == 0 && sCrm) a.crmax[c] = __longlong_as_double((long long)sCrm);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) colls += __shfl_xor_sync(kFull, colls, o);
+    if (lane == 0 && colls) atomicAdd(a.counters + C_COLLISIONS, (unsigned long long)colls);
+}
+
+// resident blocks per SM of the collision kernel, set by prepare_kernels
 template <typename Real>
 struct CellOcc {
     static int blocks;
@@ -1535,12 +1642,13 @@ int CellOcc<Real>::blocks = 1;
 template <typename Real>
 cudaError_t prepare_kernels()
 {
-    cudaError_t e = cudaFuncSetAttribute(collide_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)cell_smem_bytes<Real>());
+    constexpr size_t cellBytes = kCellWarps * arena_bytes<Real>(kArena), bigBytes = arena_bytes<Real>(kBigArena);
+    cudaError_t e = cudaFuncSetAttribute(collide_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cellBytes);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(collide_big_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bigBytes);
     if (e != cudaSuccess) return e;
     int nb = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, collide_kernel<Real>, kCellWarps * 32,
-                                                      cell_smem_bytes<Real>());
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, collide_kernel<Real>, kCellWarps * 32, cellBytes);
     if (e != cudaSuccess) return e;
     CellOcc<Real>::blocks = nb > 0 ? nb : 1;
     const void* stay[3] = {(const void*)move_stay_kernel<Real, 1>, (const void*)move_stay_kernel<Real, 2>,
@@ -1554,17 +1662,22 @@ cudaError_t prepare_kernels()
 }
 
 template <typename Real>
-void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s)
+void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s, const SideStream& side)
 {
     const int ncell = a.M.ncell;
     cudaMemsetAsync(a.cellWork, 0, 8 * sizeof(int), s);
     int gc = (ncell + 255) / 256;
     if (gc > L.smCount * 8) gc = L.smCount * 8;
-    classify_kernel<Real><<<gc > 0 ? gc : 1, 256, 0, s>>>(a, kArena);
+    classify_kernel<Real><<<gc > 0 ? gc : 1, 256, 0, s>>>(a);
+    // the big cells' kernel goes first: its blocks need much of an SM's
+    // shared memory, and the other cells' blocks fill what they leave
+    side.fork(s);
+    collide_big_kernel<Real><<<L.smCount, kBigThreads, arena_bytes<Real>(kBigArena), side.stream>>>(a);
     int g = (ncell + kCellWarps - 1) / kCellWarps;
     const int cap = L.smCount * min(CellOcc<Real>::blocks, max(1, L.collideBlocksPerSm));
     if (g > cap) g = cap;
-    collide_kernel<Real><<<g > 0 ? g : 1, kCellWarps * 32, cell_smem_bytes<Real>(), s>>>(a);
+    collide_kernel<Real><<<g > 0 ? g : 1, kCellWarps * 32, kCellWarps * arena_bytes<Real>(kArena), s>>>(a);
+    side.join(s);
 }
 
 // ===========================================================================
@@ -1978,7 +2091,7 @@ void launch_trace_check(const DevMesh& M, const DevConsts& C, int n, const Real*
     template void launch_inject<Real>(const StepArgs<Real>&, const LaunchShape&, cudaStream_t);                  \
     template void launch_move<Real>(const StepArgs<Real>&, const LaunchShape&, cudaStream_t);                    \
     template void launch_sort<Real>(const StepArgs<Real>&, const LaunchShape&, cudaStream_t);                    \
-    template void launch_collide<Real>(const StepArgs<Real>&, const LaunchShape&, cudaStream_t);                 \
+    template void launch_collide<Real>(const StepArgs<Real>&, const LaunchShape&, cudaStream_t, const SideStream&); \
     template void launch_sample<Real>(const StepArgs<Real>&, bool, const LaunchShape&, cudaStream_t);            \
     template void launch_fill<Real>(const StepArgs<Real>&, const FillParams&, const int*, const LaunchShape&,    \
                                     cudaStream_t);                                                               \

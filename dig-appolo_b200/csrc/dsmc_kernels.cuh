@@ -70,8 +70,8 @@ struct StepArgs {
     unsigned long long* counters;
     int* cellPairs;           // [ncell] candidate pair count of the step (classify pass)
     double* cellCons;         // [ncell] majorant term of the pair count (classify pass)
-    int* cellList;            // [2*ncell] work lists of the cell pass
-    int4* cellItem;           // [ncell] huge / large items at their list slot: cell, start, count, pairs
+    int* cellList;            // [2*ncell] small, big and giant cells of the collision pass
+    int4* cellItem;           // [ncell] large cells of the collision pass: cell, start, count, pairs
     double2* cellItemC;       // [ncell] the same items' majorant term and crmax
     int* cellWork;            // [8] list lengths and hand-out counters of the cell pass
     int* errorWord;
@@ -91,10 +91,31 @@ struct LaunchShape {
     int stayPerThread = 4;        // particles per thread of the move's stay pass: 1, 2 or 4
 };
 
+// A second stream for kernels that run beside those of the main stream: it
+// takes up after the work queued on the main stream at the fork, and the
+// main stream's later work follows it from the join. The same calls make a
+// branch of a graph under capture. Its priority is higher than the main
+// stream's, so its blocks are placed first.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
+    void fork(cudaStream_t main) const
+    {
+        cudaEventRecord(forked, main);
+        cudaStreamWaitEvent(stream, forked, 0);
+    }
+    void join(cudaStream_t main) const
+    {
+        cudaEventRecord(joined, stream);
+        cudaStreamWaitEvent(main, joined, 0);
+    }
+};
+
 template <typename Real> void launch_inject(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s);
 template <typename Real> void launch_move(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s);
 template <typename Real> void launch_sort(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s);
-template <typename Real> void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s);
+template <typename Real>
+void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s, const SideStream& side);
 template <typename Real> void launch_sample(const StepArgs<Real>& a, bool pre, const LaunchShape& L, cudaStream_t s);
 void launch_bump_istep(StepCtl* ctl, cudaStream_t s);
 
