@@ -710,12 +710,12 @@ __device__ __forceinline__ void sort_far_warp(int* seg, int m)
 __device__ void sort_far(int* seg, int m, int* tmp)
 {
     const int lane = threadIdx.x & 31;
-    if (m <= 1) return;
-    if (m <= 32) {
-        sort_far_warp<1>(seg, m);
-    } else if (m <= 512) {
-        sort_far_warp<16>(seg, m);
-    } else {
+    if (m <= 32) sort_far_warp<1>(seg, m);
+    else if (m <= 64) sort_far_warp<2>(seg, m);
+    else if (m <= 128) sort_far_warp<4>(seg, m);
+    else if (m <= 256) sort_far_warp<8>(seg, m);
+    else if (m <= 512) sort_far_warp<16>(seg, m);
+    else {
         // rank counting: O(m^2 / 32), for the rare very large far segments
         for (int e = lane; e < m; e += 32) tmp[e] = seg[e];
         __syncwarp();
@@ -732,11 +732,15 @@ __device__ void sort_far(int* seg, int m, int* tmp)
 // Canonical order of every cell's far-slot arrivals: ascending source
 // index; the far counts are cleared for the next step's rank pass. Each
 // lane takes one cell: a segment of up to kLaneSort arrivals (the common
-// case: multi-cell hops and injected particles are some tens per cell at
-// most) is insertion-sorted in the lane's own shared-memory row; longer
-// ones by the whole warp, whose output cell ids serve as scratch for very
-// long ones and are restored.
-constexpr int kLaneSort = 32;
+// case, multi-cell hops) is insertion-sorted in the lane's own shared-memory
+// row; longer ones (the cells behind an inlet, up to hundreds a step) by the
+// whole warp, whose output cell ids serve as scratch for very long ones and
+// are restored. A warp's 32 cells lie a grid apart: the inlet's cells are
+// neighbours in the numbering, and in consecutive order one warp had 32 of
+// them to sort one after another (6,080 hexahedra at 96 a cell: 116
+// us; 6 as it is, each with a sort of the segment's own size instead
+// of 512).
+constexpr int kLaneSort = 12;
 constexpr int kFarsortThreads = 256;
 
 __global__ void __launch_bounds__(kFarsortThreads) farsort_kernel(int* countSlot, const int* startB, int* idx,
@@ -747,15 +751,19 @@ __global__ void __launch_bounds__(kFarsortThreads) farsort_kernel(int* countSlot
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int base = warp * 32; base < ncell; base += nwarps * 32) {
-        const int c = base + lane;
-        int far = 0;
+    for (long long first = warp; first < ncell; first += 32ll * nwarps) {
+        const long long at = first + (long long)lane * nwarps;
+        const int c = at < ncell ? (int)at : ncell;
+        int far = 0, end = 0;
         if (c < ncell) {
             far = countSlot[(size_t)c * kSlots + kFarSlot];
-            if (far) countSlot[(size_t)c * kSlots + kFarSlot] = 0;
+            if (far) {
+                countSlot[(size_t)c * kSlots + kFarSlot] = 0;
+                end = startB[c + 1];
+            }
         }
         if (far >= 2 && far <= kLaneSort) {
-            int* seg = idx + startB[c + 1] - far;
+            int* seg = idx + end - far;
             for (int k = 0; k < far; ++k) row[k] = seg[k];
             for (int k = 1; k < far; ++k) {
                 const int v = row[k];
@@ -770,9 +778,9 @@ __global__ void __launch_bounds__(kFarsortThreads) farsort_kernel(int* countSlot
         }
         for (unsigned m = __ballot_sync(kFull, far > kLaneSort); m; m &= m - 1) {
             const int l = __ffs(m) - 1;
-            const int cl = base + l;
+            const int cl = __shfl_sync(kFull, c, l);
             const int f = __shfl_sync(kFull, far, l);
-            const int e = startB[cl + 1];
+            const int e = __shfl_sync(kFull, end, l);
             sort_far(idx + e - f, f, cellB + e - f);
             if (f > 512) {
                 for (int k = lane; k < f; k += 32) cellB[e - f + k] = cl;
