@@ -71,7 +71,8 @@ struct DevMesh {
     const signed char* revSlot;  // [ncell*6] slot of this cell in neighbour j's list (or -1)
     // face planes (cells with convex[c] != 0): records faceOff[c]..faceOff[c+1]
     const int* faceOff;          // [ncell+1]
-    const int4* faceRec;         // face id, index of its first triangle, node count (3/4), and the crossing:
+    const int4* faceRec;         // face id, index of its first triangle, node count (3/4) | (record slot + 1) << 8
+                                 // of the face in the cell on the other side (0: unknown), and the crossing:
                                  // the cell on the other side (interface), kNbLost, or -(role + 1)
     const float4* planeF;        // outward unit normal, offset relative to the cell centre
     const float4* diagF;         // quads: in-plane normal of the diagonal, offset (relative)
@@ -79,9 +80,12 @@ struct DevMesh {
     const unsigned char* convex; // [ncell]
     const float2* recAux;        // [nrec] x: min |e1 x e2| over the record's triangles (0 when one of them is
                                  // ill-conditioned), y: the cell's length scale (sum over axes of the
-                                 // largest node offset from the centre)
+                                 // largest node offset from the centre, plus 2^-11 of the centre's
+                                 // absolute coordinates: the rounding of an FP64 position)
+    const float4* geo;           // faceStride 4-6: per cell what a search reads, in one or two lines (CellGeo)
     int faceStride;              // F when every cell is convex with F records (record k = cell * F + j), else 0
     int allConvex;               // every cell takes the plane path
+    int triPerRec;               // 1 / 2: the first triangle of record k is k / 2 k (all faces triangles / quads), else 0
     // placement tetrahedra of each cell (buildCellInitTets): records
     // placeOff[c]..placeOff[c+1], four vertices each (absolute FP64; the
     // barycentric weights a, b, c, d go to them in this order) and volume
@@ -339,7 +343,7 @@ __device__ __forceinline__ ExitHit find_exit_exact(const DevMesh& M, int cell, i
 
 // ---------------------------------------------------------------------------
 // Plane-based exit search of the FP64 path, for cells that are convex with
-// planar faces.
+// planar faces, where the FP32 test below settles nothing.
 //
 // The exit of a ray from inside a convex cell is the face plane it reaches
 // first among those it moves towards: t_f = (d_f - n_f.x) / (v.n_f) for
@@ -408,7 +412,7 @@ __device__ __forceinline__ PlaneHit find_exit_planes(const DevMesh& M, int cell,
     h.tri = -1;
     h.triIdx = rec.y;
     h.nb = rec.w;
-    if (rec.z == 4) {
+    if ((rec.z & 0xff) == 4) {
         const double* pd = M.planeD + (size_t)bi * 8;
         const double mx = pd[4], my = pd[5], mz = pd[6], md = pd[7];
         const double px = x[0] + v[0] * best, py = x[1] + v[1] * best, pz = x[2] + v[2] * best;
@@ -423,9 +427,10 @@ __device__ __forceinline__ PlaneHit find_exit_planes(const DevMesh& M, int cell,
 }
 
 // ---------------------------------------------------------------------------
-// The mixed path's exit test: FP32 arithmetic that settles, where it can, what
-// the reference's FP64 triangle scan (find_exit_exact) returns, so that the
-// mixed trace takes the same decisions as the FP64 trace.
+// The exit test: FP32 arithmetic that settles, where it can, what the
+// reference's FP64 triangle scan (find_exit_exact) returns, so that the
+// mixed trace takes the same decisions as the FP64 trace, and the FP64 trace
+// takes them at FP32 cost.
 //
 // Inputs: the position relative to the cell centre rounded to FP32 from the
 // trace's FP64 position, the FP32 velocity, and the cell's FP32 face planes.
@@ -452,101 +457,164 @@ __device__ __forceinline__ PlaneHit find_exit_planes(const DevMesh& M, int cell,
 // Then the reference's scan returns f (with the half `tri`) at a t inside
 // [tLo, tHi]. Anything else is not certain and the caller runs that scan.
 // ---------------------------------------------------------------------------
+// What the test reads of a cell: its face planes, the smallest |e1 x e2| of
+// each record's triangles and the length scale, and for the trace around it
+// the centre. kFaces > 0: from one block per cell (128 bytes for 4 and 5
+// faces, 160 for 6), which a particle entering the cell misses once instead
+// of in three arrays; the planes, the centre (3 doubles), the scale, the
+// kFaces determinants. Else from the mesh's arrays.
+template <int kFaces>
+struct CellGeo {
+    static constexpr int kFloats = kFaces == 6 ? 40 : 32;
+    const float4* at;
+    __device__ __forceinline__ CellGeo(const DevMesh& M, int cell, int, int)
+        : at(M.geo + (size_t)cell * (kFloats / 4))
+    {
+    }
+    __device__ __forceinline__ float4 plane(int k) const { return at[k]; }
+    __device__ __forceinline__ const double* centre() const { return reinterpret_cast<const double*>(at + kFaces); }
+    __device__ __forceinline__ float scale() const { return reinterpret_cast<const float*>(at + kFaces)[6]; }
+    __device__ __forceinline__ float det(int k) const { return reinterpret_cast<const float*>(at + kFaces)[7 + k]; }
+};
+template <>
+struct CellGeo<0> {
+    const float4* planes;
+    const float2* aux;
+    const double* cc;
+    bool any;
+    __device__ __forceinline__ CellGeo(const DevMesh& M, int cell, int b, int faces)
+        : planes(M.planeF + b), aux(M.recAux + b), cc(M.cellCenter + (size_t)cell * 3), any(faces > 0)
+    {
+    }
+    __device__ __forceinline__ float4 plane(int k) const { return planes[k]; }
+    __device__ __forceinline__ const double* centre() const { return cc; }
+    __device__ __forceinline__ float scale() const { return any ? aux[0].y : 0.0f; }
+    __device__ __forceinline__ float det(int k) const { return aux[k].x; }
+};
+template <int kFaces>
+__device__ __forceinline__ const double* cell_centre(const DevMesh& M, int cell)
+{
+    if constexpr (kFaces > 0) return CellGeo<kFaces>(M, cell, 0, 0).centre();
+    else return M.cellCenter + (size_t)cell * 3;
+}
+
 struct CertainExit {
     bool certain;
     int face, tri, triIdx;
     int nb;        // the record's crossing (as PlaneHit::nb)
+    int slot, rev; // the face's record within this cell, and within the cell on the other side (-2: unknown)
     float tLo, tHi;
 };
 
 constexpr float kEps32 = 5.9604645e-8f;   // 2^-24
 
-// kAtRest: the search of a particle at rest in its cell (crossf -1, as in
-// the stay pass), which has no entry face and reads no face records in its
-// loop; the same result as the general form with crossf -1.
+// entry: the entry face's record within the cell, -1 at rest in the cell
+// (no entry face), -2 unknown (crossf is then looked up in the face records).
+// kAtRest: the search of a particle at rest in its cell (entry -1, as in the
+// stay pass); the same result as the general form with entry -1.
 // kFaces > 0: the mesh's face records sit at cell * kFaces (faceStride ==
-// kFaces, checked by the caller), and the face loop is unrolled with its
-// loads issued together.
-template <bool kAtRest = false, int kFaces = 0>
-__device__ __forceinline__ CertainExit certain_exit_f32(const DevMesh& M, int cell, int crossf, int tag,
-                                                        const float x[3], const float v[3], float absScale)
+// kFaces, checked by the caller), the face loop is unrolled, and what it reads
+// of the cell lies together (CellGeo). The loop reads the planes only (the
+// entry face comes as a record slot, not by its id), and the records of the
+// face chosen and its triangle are then read together, so a search waits for
+// two round trips to memory: the cell, then the chosen face.
+// One division a face: each bound of t is over v.n + vErr but tHi's, which
+// only the face chosen needs.
+template <bool kAtRest, int kFaces>
+__device__ __forceinline__ CertainExit certain_exit_f32(const DevMesh& M, int cell, int crossf, int entry, int tag,
+                                                        const float x[3], const float v[3])
 {
-    CertainExit r{false, -2, -1, -1, 0, 0.0f, 0.0f};
+    CertainExit r{false, -2, -1, -1, 0, -1, -2, 0.0f, 0.0f};
     const float vnorm = fabsf(v[0]) + fabsf(v[1]) + fabsf(v[2]);
     const float xnorm = fabsf(x[0]) + fabsf(x[1]) + fabsf(x[2]);
     const float vErr = 32.0f * kEps32 * vnorm;
-    const float absErr = 0x1p-30f * absScale;
     const int b = kFaces ? cell * kFaces : (M.faceStride ? cell * M.faceStride : M.faceOff[cell]);
-    const int e = kFaces ? b + kFaces : (M.faceStride ? b + M.faceStride : M.faceOff[cell + 1]);
+    const int faces = kFaces ? kFaces : (M.faceStride ? M.faceStride : M.faceOff[cell + 1] - b);
+    if constexpr (!kAtRest) {
+        if (entry == -2) {
+            for (int k = 0; k < faces; ++k)
+                if (M.faceRec[b + k].x == crossf) { entry = k; break; }
+            if (entry == -2) return r;
+        }
+    }
     int bi = -1;
-    float best = FLT_MAX, bestLo = 0.0f, bestHi = 0.0f, bestTau = 0.0f, bestVn = 0.0f;
+    float best = FLT_MAX, bestNum = 0.0f, bestDErr = 0.0f, bestTau = FLT_MAX, bestVn = 0.0f;
     float tauMin = FLT_MAX;   // latest t_f every other approached face allows
     float entA = 0.0f, entB = 0.0f;
     bool ok = true;
+    const CellGeo<kFaces> geo(M, cell, b, faces);
     // the length scale is the cell's (the same in each of its records)
-    const float lc = b < e ? M.recAux[b].y : 0.0f;
-    const float dErr0 = 32.0f * kEps32 * (xnorm + lc) + absErr;
+    const float lc = geo.scale();
+    const float dErr0 = 32.0f * kEps32 * (xnorm + lc);
 #pragma unroll(kFaces > 0 ? kFaces : 1)
-    for (int k = b; k < e; ++k) {
-        int4 rec = make_int4(-1, 0, 0, 0);
-        if constexpr (!kAtRest) rec = M.faceRec[k];
-        const float4 pl = M.planeF[k];
+    for (int k = 0; k < faces; ++k) {
+        const float4 pl = geo.plane(k);
         const float vn = v[0] * pl.x + v[1] * pl.y + v[2] * pl.z;
         const float num = pl.w - (x[0] * pl.x + x[1] * pl.y + x[2] * pl.z);
         const float dErr = 32.0f * kEps32 * fabsf(pl.w) + dErr0;
-        if (!kAtRest && rec.x == crossf) {
+        const bool isEntry = !kAtRest && k == entry;
+        if (isEntry) {
             // entry face: moving away from it; its edge with the exit face is
             // checked below (slack entA + t_f * entB)
-            if (!(vn < -vErr)) ok = false;
+            ok = ok && vn < -vErr;
             entA = num - 2.0f * dErr;
             entB = -vn - vErr;
-            if (rec.z == 4 && (tag == 1 || tag == 2)) {
-                const float4 dg = M.diagF[k];
+            if (tag == 1 || tag == 2) {   // the half of a quad
+                const float4 dg = M.diagF[b + k];
                 const float side = dg.x * x[0] + dg.y * x[1] + dg.z * x[2] - dg.w;
-                const float sErr = 2.0f * (32.0f * kEps32 * (fabsf(dg.w) + xnorm + lc) + absErr);
-                if (!(tag == 1 ? side > sErr : side < -sErr)) ok = false;
+                const float sErr = 64.0f * kEps32 * (fabsf(dg.w) + xnorm + lc);
+                ok = ok && (tag == 1 ? side > sErr : side < -sErr);
             }
-            continue;
-        }
-        if (!(num > 2.0f * dErr) || !(fabsf(vn) > vErr)) { ok = false; continue; }
-        if (vn < 0.0f) continue;   // left behind: never reached
-        // fast divisions (a few ulp, well inside dErr's margin), each bound
-        // then moved outwards by 2^-21 of itself
-        const float t = __fdividef(num, vn);
-        const float tLo = __fdividef(num - dErr, vn + vErr) * (1.0f - 0x1p-21f);
-        const float tHi = __fdividef(num + dErr, vn - vErr) * (1.0f + 0x1p-21f);
-        const float tau = __fdividef(num - 2.0f * dErr, vn + vErr) * (1.0f - 0x1p-21f);
-        if (t < best) {
-            if (bi >= 0) tauMin = fminf(tauMin, bestTau);
-            best = t; bestLo = tLo; bestHi = tHi; bestTau = tau; bestVn = vn; bi = k;
         } else {
-            tauMin = fminf(tauMin, tau);
+            ok = ok && num > 2.0f * dErr && fabsf(vn) > vErr;
+        }
+        // a face left behind is never reached
+        const bool reached = !isEntry && vn > 0.0f;
+        // fast reciprocal (with the product a few ulp, well inside dErr's
+        // margin), each bound then moved outwards by 2^-20 of itself
+        const float rv = __fdividef(1.0f, vn + vErr);
+        const float t = reached ? num * rv : FLT_MAX;
+        const float tau = reached ? (num - 2.0f * dErr) * rv * (1.0f - 0x1p-20f) : FLT_MAX;
+        const bool first = t < best;
+        tauMin = fminf(tauMin, first ? bestTau : tau);
+        if (first) {
+            best = t; bestNum = num; bestDErr = dErr; bestTau = tau; bestVn = vn; bi = k;
         }
     }
     if (!ok || bi < 0) return r;
+    const float bestLo = __fdividef(bestNum - bestDErr, bestVn + vErr) * (1.0f - 0x1p-20f);
+    const float bestHi = __fdividef(bestNum + bestDErr, bestVn - vErr) * (1.0f + 0x1p-20f);
     if (!(bestHi < tauMin)) return r;
-    if (crossf >= 0 && !(entA + bestLo * entB > 0.0f)) return r;
-    const float2 aux = M.recAux[bi];
-    if (!(bestVn >= 0x1p-10f * vnorm)) return r;            // grazing exit
-    if (!((bestVn - vErr) * aux.x > 2e-14f)) return r;       // |det| near the 1e-14 cut, or ill-conditioned
+    if (!kAtRest && entry >= 0 && !(entA + bestLo * entB > 0.0f)) return r;
+    if (!(bestVn >= 0x1p-10f * vnorm)) return r;             // grazing exit
     if (!(bestLo > 2e-14f)) return r;                        // the reference's t > 1e-14
-    const int4 rec = M.faceRec[bi];
-    int tri = -1, triIdx = rec.y;
-    if (rec.z == 4) {
-        const float4 dg = M.diagF[bi];
+    if (!((bestVn - vErr) * geo.det(bi) > 2e-14f)) return r; // |det| near the 1e-14 cut, or ill-conditioned
+    // where all faces are triangles, a search at rest needs no record: only
+    // whether the exit is certain, and when
+    if (kAtRest && M.triPerRec == 1) {
+        r.certain = true;
+        r.tLo = bestLo;
+        return r;
+    }
+    const int4 rec = M.faceRec[b + bi];
+    int tri = -1, triIdx = M.triPerRec ? (b + bi) * M.triPerRec : rec.y;
+    if ((rec.z & 0xff) == 4) {
+        const float4 dg = M.diagF[b + bi];
         const float px = x[0] + v[0] * best, py = x[1] + v[1] * best, pz = x[2] + v[2] * best;
         const float side = dg.x * px + dg.y * py + dg.z * pz - dg.w;
-        const float sErr = 32.0f * kEps32 * (fabsf(dg.w) + fabsf(px) + fabsf(py) + fabsf(pz) + aux.y) + absErr +
+        const float sErr = 32.0f * kEps32 * (fabsf(dg.w) + fabsf(px) + fabsf(py) + fabsf(pz) + lc) +
                            vnorm * (bestHi - bestLo);
         if (!(fabsf(side) > 2.0f * sErr)) return r;
         tri = side > 0.0f ? 1 : 2;
-        triIdx = rec.y + (tri == 2 ? 1 : 0);
+        triIdx += tri == 2 ? 1 : 0;
     }
     r.certain = true;
     r.face = rec.x;
     r.tri = tri;
     r.triIdx = triIdx;
     r.nb = rec.w;
+    r.slot = bi;
+    r.rev = (rec.z >> 8) ? (rec.z >> 8) - 1 : -2;
     r.tLo = bestLo;
     r.tHi = bestHi;
     return r;
@@ -565,6 +633,23 @@ struct PRegs {
     Real v[3];
     Real ir;
 };
+
+// certain_exit_f32 for a particle in registers: its FP32 offset from the
+// cell's centre and FP32 velocity. An FP64 velocity is rounded for the test
+// (one ulp of each component, within vErr's margin over the roundings of
+// v.n), so the FP64 path takes the same decision at FP32 cost; a speed whose
+// error bound could underflow settles nothing.
+template <typename Real, bool kAtRest, int kFaces>
+__device__ __forceinline__ CertainExit search_certain(const DevMesh& M, int cell, int crossf, int entry, int tag,
+                                                      const PRegs<Real>& p)
+{
+    const double* cc = cell_centre<kFaces>(M, cell);
+    const float xr[3] = {(float)ds(p.x[0], cc[0]), (float)ds(p.x[1], cc[1]), (float)ds(p.x[2], cc[2])};
+    const float v[3] = {(float)p.v[0], (float)p.v[1], (float)p.v[2]};
+    CertainExit ce = certain_exit_f32<kAtRest, kFaces>(M, cell, crossf, entry, tag, xr, v);
+    if constexpr (sizeof(Real) == 8) ce.certain = ce.certain && fabsf(v[0]) + fabsf(v[1]) + fabsf(v[2]) > 1e-20f;
+    return ce;
+}
 
 struct TraceLog {        // optional per-particle record for the tracing check
     int hitFace;
@@ -654,14 +739,18 @@ struct TraceState {
     int ifout;        // outcome so far
     int iter;         // exit searches made
     int crossf, tag;  // the face / triangle the particle entered through
+    int entry;        // that face's record within the cell (-1 none, -2 not known)
     bool afterNone;   // the last hit had no handler: use the triangle search
+    bool scan;        // the search left the exit to the triangle scan, to be run by the warp (kWarpScan)
     __device__ __forceinline__ void begin(int crossf0, int tag0)
     {
         ifout = kTraceStay;
         iter = 0;
         crossf = crossf0;
         tag = tag0;
+        entry = crossf0 >= 0 ? -2 : -1;
         afterNone = false;
+        scan = false;
     }
 };
 
@@ -670,83 +759,102 @@ struct TraceState {
 // the step or the crossing with its boundary handling. Returns true when the
 // trace is over, with the outcome in st.ifout.
 //
-// Exit search. FP64 path: the FP64 plane decision confirmed by the
-// reference's test on the chosen triangle, else the reference's triangle
-// scan. Mixed path: certain_exit_f32 on the FP32 offsets; a certain exit
-// beyond the rest of the step needs no FP64 test at all (the particle stays),
-// a certain crossing takes its t from the reference's FP64 test on the one
-// triangle it names, and everything else runs the reference's FP64 triangle
-// scan (counter `fp64_fallbacks`). Positions, dtleft and every decision are
-// then those of the FP64 trace from the same stored state; only wall
-// re-emission draws FP32 velocities.
-template <typename Real, typename Rng>
+// Exit search, both paths: certain_exit_f32 on the FP32 offsets; a certain
+// exit beyond the rest of the step needs no FP64 test at all (the particle
+// stays), and a certain crossing takes its t from the reference's FP64 test on
+// the one triangle it names. What that does not settle: on the FP64 path the
+// FP64 plane decision confirmed by the reference's test on the chosen
+// triangle, and else, on the mixed path at once (counter `fp64_fallbacks`),
+// the reference's FP64 triangle scan. Positions, dtleft and every decision of
+// the mixed path are then those of the FP64 trace from the same stored state;
+// only wall re-emission draws FP32 velocities.
+//
+// kWarpScan: a search that needs the triangle scan sets st.scan and leaves
+// the particle as it is; before the next pass the warp runs the scan
+// (scan_pending), and that pass takes its result from *scanned. The injection
+// traces so, one latency chain on few SMs (6,080 hexahedra: 115 -> 92 us). In
+// the tracing pass of the move the registers it takes cost more than the
+// scans (372,500 tetrahedra: 918 against 1058 us), so a lane scans alone.
+template <typename Real, typename Rng, int kFaces, bool kWarpScan>
 __device__ __forceinline__ bool trace_step(const DevMesh& M, const DevConsts& C, PRegs<Real>& p, int& cell,
                                            double& dtleft, TraceState& st, Rng& rng, int istep,
-                                           double* wallTally, TraceCounts& cnt, bool stopAtWall, TraceLog* log)
+                                           double* wallTally, TraceCounts& cnt, bool stopAtWall, TraceLog* log,
+                                           const ExitHit* scanned = nullptr)
 {
     int& ifout = st.ifout;
     int& crossf = st.crossf;
     int& tag = st.tag;
     bool& afterNone = st.afterNone;
-    if (!(dtleft > 0.0)) return true;
-    if (st.iter++ >= C.maxCross) { cnt.lost++; dtleft = 0; ifout = kTraceLost; return true; }
+    const bool haveScan = kWarpScan && st.scan;
+    if (!haveScan) {
+        if (!(dtleft > 0.0)) return true;
+        if (st.iter++ >= C.maxCross) { cnt.lost++; dtleft = 0; ifout = kTraceLost; return true; }
+    }
     int face = -2, tri = -1;
     double t = 0.0;
     bool decided = false;
     int hintNb = 0;   // a face chosen from a face record comes with the record's crossing
-    if ((M.allConvex || M.convex[cell]) && !afterNone) {
-        if constexpr (sizeof(Real) == 8) {
-            // plane decision, then the reference's exact test on that one
-            // triangle for the bit-exact t; any doubt runs the full search
-            const PlaneHit ph = find_exit_planes(M, cell, crossf, p.x, p.v);
-            double te = DBL_MAX;
-            if (!ph.ambiguous && isect_exact(M.triD + (size_t)ph.triIdx * 9, p.x, p.v, te)) {
-                face = ph.face; tri = ph.tri; t = te;
-                decided = true;
-                hintNb = ph.nb;
-                // the other half of a quad entry face stays eligible in
-                // the reference's skip rule (src/ProcessDSMC.cpp:1229-1233)
-                if (crossf >= 0 && (tag == 1 || tag == 2)) {
-                    const int b0 = M.triOffset[cell], e0 = M.triOffset[cell + 1];
-                    for (int k = b0; k < e0; ++k) {
-                        const int2 ft = M.triFT[k];
-                        if (ft.x != crossf || ft.y == tag || ft.y <= 0) continue;
-                        double t2 = DBL_MAX;
-                        if (isect_exact(M.triD + (size_t)k * 9, p.x, p.v, t2) && t2 < t) decided = false;
-                    }
-                }
+    int slot = -2, rev = -2;   // and its record within this cell and within the next
+    if (!haveScan && (M.allConvex || M.convex[cell]) && !afterNone) {
+        const CertainExit ce = search_certain<Real, false, kFaces>(M, cell, crossf, st.entry, tag, p);
+        if (ce.certain) {
+            if (ce.tLo > (float)dtleft * (1.0f + 0x1p-16f)) {
+                // the reference's scan would return this face at t >= dtleft
+                advance(p, dtleft);
+                dtleft = 0;
+                return true;
             }
-        } else {
-            const double* cc = M.cellCenter + (size_t)cell * 3;
-            const double c0 = cc[0], c1 = cc[1], c2 = cc[2];
-            const float xr[3] = {(float)ds(p.x[0], c0), (float)ds(p.x[1], c1), (float)ds(p.x[2], c2)};
-            const float absScale = (float)(fabs(c0) + fabs(c1) + fabs(c2));
-            const CertainExit ce = M.faceStride == 4
-                                       ? certain_exit_f32<false, 4>(M, cell, crossf, tag, xr, p.v, absScale)
-                                       : certain_exit_f32<false, 0>(M, cell, crossf, tag, xr, p.v, absScale);
-            if (ce.certain) {
-                if (ce.tLo > (float)dtleft * (1.0f + 0x1p-16f)) {
-                    // the reference's scan would return this face at t >= dtleft
-                    advance(p, dtleft);
-                    dtleft = 0;
-                    return true;
-                }
-                const double v64[3] = {(double)p.v[0], (double)p.v[1], (double)p.v[2]};
+            const double v64[3] = {(double)p.v[0], (double)p.v[1], (double)p.v[2]};
+            double te = DBL_MAX;
+            if (isect_exact(M.triD + (size_t)ce.triIdx * 9, p.x, v64, te)) {
+                face = ce.face; tri = ce.tri; t = te;
+                decided = true;
+                hintNb = ce.nb;
+                slot = ce.slot;
+                rev = ce.rev;
+            }
+        }
+        if constexpr (sizeof(Real) == 8) {
+            // what FP32 cannot settle: the FP64 plane decision, then the
+            // reference's exact test on that one triangle for the bit-exact
+            // t; any doubt runs the full search
+            if (!decided) {
+                const PlaneHit ph = find_exit_planes(M, cell, crossf, p.x, p.v);
                 double te = DBL_MAX;
-                if (isect_exact(M.triD + (size_t)ce.triIdx * 9, p.x, v64, te)) {
-                    face = ce.face; tri = ce.tri; t = te;
+                if (!ph.ambiguous && isect_exact(M.triD + (size_t)ph.triIdx * 9, p.x, p.v, te)) {
+                    face = ph.face; tri = ph.tri; t = te;
                     decided = true;
-                    hintNb = ce.nb;
+                    hintNb = ph.nb;
+                    // the other half of a quad entry face stays eligible in
+                    // the reference's skip rule (src/ProcessDSMC.cpp:1229-1233)
+                    if (crossf >= 0 && (tag == 1 || tag == 2)) {
+                        const int b0 = M.triOffset[cell], e0 = M.triOffset[cell + 1];
+                        for (int k = b0; k < e0; ++k) {
+                            const int2 ft = M.triFT[k];
+                            if (ft.x != crossf || ft.y == tag || ft.y <= 0) continue;
+                            double t2 = DBL_MAX;
+                            if (isect_exact(M.triD + (size_t)k * 9, p.x, p.v, t2) && t2 < t) decided = false;
+                        }
+                    }
                 }
             }
         }
     }
-    if constexpr (sizeof(Real) == 4) {
-        if (!decided) cnt.fallback++;
-    }
     if (!decided) {
-        const double v64[3] = {(double)p.v[0], (double)p.v[1], (double)p.v[2]};
-        const ExitHit h = find_exit_exact(M, cell, crossf, tag, p.x, v64);
+        ExitHit h;
+        if constexpr (kWarpScan) {
+            if (!haveScan) {
+                if constexpr (sizeof(Real) == 4) cnt.fallback++;
+                st.scan = true;
+                return false;
+            }
+            st.scan = false;
+            h = *scanned;
+        } else {
+            if constexpr (sizeof(Real) == 4) cnt.fallback++;
+            const double v64[3] = {(double)p.v[0], (double)p.v[1], (double)p.v[2]};
+            h = find_exit_exact(M, cell, crossf, tag, p.x, v64);
+        }
         if (h.face == -2 || !isfinite(h.t) || h.t <= 0.0) { cnt.dropped++; dtleft = 0; ifout = kTraceDropped; return true; }
         face = h.face; tri = h.tri; t = h.t;
     }
@@ -757,6 +865,7 @@ __device__ __forceinline__ bool trace_step(const DevMesh& M, const DevConsts& C,
     }
     crossf = face;
     tag = tri;
+    st.entry = slot;
     const int role = !decided ? (int)M.faceRole[face] : (hintNb >= 0 || hintNb == kNbLost) ? kRoleInterface : -(hintNb + 1);
     if (log && role != kRoleInterface && log->hitFace < 0) {
         log->hitFace = face;
@@ -776,6 +885,7 @@ __device__ __forceinline__ bool trace_step(const DevMesh& M, const DevConsts& C,
         ifout = kTraceMoved;
         dtleft = ds(dtleft, t);
         int next;
+        st.entry = rev;
         if (decided) {
             next = hintNb;
         } else {
@@ -818,29 +928,96 @@ __device__ __forceinline__ bool trace_step(const DevMesh& M, const DevConsts& C,
     return false;
 }
 
+// find_exit_exact by a warp, one triangle a lane, the same arguments in all
+// lanes: the nearest hit, of equal ones the first.
+static __device__ __noinline__ ExitHit scan_exit_warp(const int* triOffset, const int2* triFT, const double* triD,
+                                                      int cell, int crossf, int prevTri, double x0, double x1,
+                                                      double x2, double v0, double v1, double v2)
+{
+    constexpr unsigned full = 0xffffffffu;
+    const double x[3] = {x0, x1, x2}, v[3] = {v0, v1, v2};
+    const int b = triOffset[cell], n = triOffset[cell + 1] - b;
+    double best = DBL_MAX;
+    int at = -1;
+    for (int k = threadIdx.x & 31; k < n; k += 32) {
+        const int2 ft = triFT[b + k];
+        if (ft.x == crossf && (ft.y <= 0 || (prevTri != 1 && prevTri != 2) || ft.y == prevTri)) continue;
+        double t = DBL_MAX;
+        if (isect_exact(triD + (size_t)(b + k) * 9, x, v, t) && t < best) {
+            best = t;
+            at = k;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double t = __shfl_xor_sync(full, best, o);
+        const int k = __shfl_xor_sync(full, at, o);
+        if (k >= 0 && (at < 0 || t < best || (t == best && k < at))) {
+            best = t;
+            at = k;
+        }
+    }
+    const int2 ft = at >= 0 ? triFT[b + at] : make_int2(-2, -1);
+    return ExitHit{ft.x, ft.y, best};
+}
+
+// The triangle scans that lanes of the warp wait for (st.scan), by the warp,
+// a triangle per lane, one such lane after another; *out is the lane's
+// result. Alone a scan is a chain of up to 12 triangle tests that the whole
+// warp waits for, about 9 us; 2e-4 to 1e-3 of the searches need one. More than
+// kScanTogether lanes at once scan side by side instead. All 32 lanes call it,
+// between two passes, where the fewest registers are in use.
+constexpr int kScanTogether = 8;
+
+template <typename Real>
+__device__ __forceinline__ void scan_pending(bool active, const DevMesh& M, const PRegs<Real>& p, int cell,
+                                             const TraceState& st, ExitHit* out)
+{
+    constexpr unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool mine = active && st.scan;
+    unsigned scans = __ballot_sync(full, mine);
+    if (scans == 0u) return;
+    if (__popc(scans) > kScanTogether) {
+        const double v64[3] = {(double)p.v[0], (double)p.v[1], (double)p.v[2]};
+        if (mine) *out = find_exit_exact(M, cell, st.crossf, st.tag, p.x, v64);
+        return;
+    }
+    for (; scans; scans &= scans - 1) {
+        const int l = __ffs(scans) - 1;
+        const ExitHit h = scan_exit_warp(
+            M.triOffset, M.triFT, M.triD, __shfl_sync(full, cell, l), __shfl_sync(full, st.crossf, l),
+            __shfl_sync(full, st.tag, l), __shfl_sync(full, p.x[0], l), __shfl_sync(full, p.x[1], l),
+            __shfl_sync(full, p.x[2], l), (double)__shfl_sync(full, p.v[0], l), (double)__shfl_sync(full, p.v[1], l),
+            (double)__shfl_sync(full, p.v[2], l));
+        if (lane == l) *out = h;
+    }
+}
+
 // The first exit search of a particle at rest in `cell` at the start of the
 // step (no entry face), taken only when it settles that the particle stays
 // in its cell for the whole of dtleft: the decision trace_step takes on that
 // search, without the triangle scan. The caller then advances it by dtleft.
-// FP64 path: the plane decision and the reference's test on the chosen
-// triangle; mixed path: certain_exit_f32.
-template <typename Real>
-__device__ __forceinline__ bool stays_for_the_step(const DevMesh& M, int cell, const PRegs<Real>& p, double dtleft)
+// certain_exit_f32, and on the FP64 path, where that settles nothing, the
+// FP64 plane decision and the reference's test on the chosen triangle.
+// xs: the stored position. The mixed path's FP32 offset is searched as it is
+// (the position it widens to differs by the rounding of an FP64 coordinate,
+// which the length scale covers), so the search does not wait for the centre.
+template <typename Real, int kFaces>
+__device__ __forceinline__ bool stays_for_the_step(const DevMesh& M, int cell, const Real xs[3], const PRegs<Real>& p,
+                                                   double dtleft)
 {
     if (!(M.allConvex || M.convex[cell])) return false;
+    CertainExit ce;
+    if constexpr (sizeof(Real) == 4) ce = certain_exit_f32<true, kFaces>(M, cell, -1, -1, -1, xs, p.v);
+    else ce = search_certain<Real, true, kFaces>(M, cell, -1, -1, -1, p);
+    if (ce.certain) return ce.tLo > (float)dtleft * (1.0f + 0x1p-16f);
     if constexpr (sizeof(Real) == 8) {
         const PlaneHit ph = find_exit_planes(M, cell, -1, p.x, p.v);
         double te = DBL_MAX;
         return !ph.ambiguous && isect_exact(M.triD + (size_t)ph.triIdx * 9, p.x, p.v, te) && te >= dtleft;
-    } else {
-        const double* cc = M.cellCenter + (size_t)cell * 3;
-        const double c0 = cc[0], c1 = cc[1], c2 = cc[2];
-        const float xr[3] = {(float)ds(p.x[0], c0), (float)ds(p.x[1], c1), (float)ds(p.x[2], c2)};
-        const float absScale = (float)(fabs(c0) + fabs(c1) + fabs(c2));
-        const CertainExit ce = M.faceStride == 4 ? certain_exit_f32<true, 4>(M, cell, -1, -1, xr, p.v, absScale)
-                                                 : certain_exit_f32<true, 0>(M, cell, -1, -1, xr, p.v, absScale);
-        return ce.certain && ce.tLo > (float)dtleft * (1.0f + 0x1p-16f);
     }
+    return false;
 }
 
 // Trace one particle, starting in `cell` having entered through face
@@ -854,7 +1031,25 @@ __device__ int trace_particle(const DevMesh& M, const DevConsts& C, PRegs<Real>&
 {
     TraceState st;
     st.begin(crossf, tag);
-    while (!trace_step<Real, Stream>(M, C, p, cell, dtleft, st, rng, istep, wallTally, cnt, stopAtWall, log)) {
+    while (!trace_step<Real, Stream, 0, false>(M, C, p, cell, dtleft, st, rng, istep, wallTally, cnt, stopAtWall, log)) {
+    }
+    return st.ifout;
+}
+
+// trace_particle for the 32 lanes of a warp together; scanned: the lane's
+// slot for a triangle scan's result.
+template <typename Real, int kFaces>
+__device__ __forceinline__ int trace_particle_warp(bool active, const DevMesh& M, const DevConsts& C, PRegs<Real>& p,
+                                                   int& cell, int crossf, int tag, double& dtleft, Stream& rng,
+                                                   int istep, double* wallTally, TraceCounts& cnt, ExitHit* scanned)
+{
+    TraceState st;
+    st.begin(crossf, tag);
+    while (__any_sync(0xffffffffu, active)) {
+        scan_pending(active, M, p, cell, st, scanned);
+        if (active && trace_step<Real, Stream, kFaces, true>(M, C, p, cell, dtleft, st, rng, istep, wallTally, cnt,
+                                                             false, nullptr, scanned))
+            active = false;
     }
     return st.ifout;
 }

@@ -695,7 +695,8 @@ struct Engine {
                 for (int q = 0; q < 3; ++q)
                     for (int d = 0; d < 3; ++d) lmax[d] = std::max(lmax[d], std::fabs(P[q][d] - cc[d]));
             }
-            const float lscale = (float)((lmax[0] + lmax[1] + lmax[2]) * (1.0 + 1e-6));
+            const double cAbs = std::fabs(cc[0]) + std::fabs(cc[1]) + std::fabs(cc[2]);
+            const float lscale = (float)((lmax[0] + lmax[1] + lmax[2] + 0x1p-11 * cAbs) * (1.0 + 1e-6));
             for (int k = faceOff[(size_t)lc]; k < faceOff[(size_t)lc + 1]; ++k) {
                 const int4 rec = faceRec[(size_t)k];
                 double detMin = DBL_MAX;
@@ -719,6 +720,11 @@ struct Engine {
         for (int lc = 0; lc < ncell && faceStride; ++lc)
             if (faceOff[(size_t)lc] != lc * faceStride) faceStride = 0;
 
+        // triangles of record k at k (all faces triangles) or 2 k (all quads)
+        int triPerRec = faceRec.empty() ? 0 : faceRec[0].z - 2;
+        for (size_t k = 0; k < faceRec.size() && triPerRec; ++k)
+            if (faceRec[k].z - 2 != triPerRec || faceRec[k].y != (int)k * triPerRec) triPerRec = 0;
+
         // --- neighbour slots for the counting sort
         std::vector<int> c2c((size_t)ncell * 6, -1);
         std::vector<signed char> rev((size_t)ncell * 6, -1);
@@ -736,6 +742,16 @@ struct Engine {
                     if (cells[(size_t)nb].cell2face[p] == f) { rev[(size_t)c * 6 + j] = (signed char)p; break; }
             }
         }
+
+        // --- with each face record, the face's record in the cell on the
+        //     other side, so the trace knows its entry face there without
+        //     comparing face ids
+        for (int lc = 0; lc < ncell; ++lc)
+            for (int k = faceOff[(size_t)lc]; k < faceOff[(size_t)lc + 1]; ++k) {
+                const int j = k - faceOff[(size_t)lc], nb = faceRec[(size_t)k].w;
+                const int p = rev[(size_t)lc * 6 + j];
+                if (nb >= 0 && p >= 0 && c2c[(size_t)lc * 6 + j] == nb) faceRec[(size_t)k].z |= (p + 1) << 8;
+            }
 
         // --- inlet emit patches: rebuildBoundaryEmitCache, src/ProcessDSMC.cpp:583-768
         if (!buildPatches()) return false;
@@ -786,6 +802,7 @@ struct Engine {
         M.convex = dConvex; M.recAux = dRecAux;
         M.faceStride = faceStride;
         M.allConvex = nconvex == ncell ? 1 : 0;
+        M.triPerRec = triPerRec;
         if (!upload(dTriOffset, triOffset) || !upload(dTriD, triD) || !upload(dTriFT, triFT) ||
             !upload(dRole, roleU8) || !upload(dFaceCells, faceCells) ||
             !upload(dFaceWall, faceWallHost) || !upload(dWallRot, wallRot) || !upload(dWallRotF, wallRotF) ||
@@ -796,6 +813,13 @@ struct Engine {
         M.faceRole = dRole; M.faceCells = dFaceCells; M.faceWall = dFaceWall;
         M.wallRot = dWallRot; M.wallRotF = dWallRotF; M.cellCenter = dCenter; M.cellVolume = dVol;
         M.cell2cell = dC2c; M.revSlot = dRev;
+        // the searches' block of each cell, packed on the device
+        if (const size_t floats = geo_floats(M)) {
+            float4* dGeo;
+            if (!alloc(dGeo, (size_t)ncell * (floats / 4), false)) return false;
+            launch_pack_geo(M, dGeo, stream);
+            M.geo = dGeo;
+        }
         {
             std::vector<double> placeV;
             buildPlacement(placeV);
@@ -972,6 +996,8 @@ struct Engine {
             !upload(dRot, rot) || !upload(dGas, gas) || !upload(dAdd, addBase) || !alloc(dCount, (size_t)np) ||
             !alloc(dStart, (size_t)np))
             return false;
+        const double sum = std::accumulate(addBase.begin(), addBase.end(), 0.0) + np;
+        P.expected = (int)std::min(sum, 1.0e9);
         P.npatch = np; P.ngroup = ngroup; P.groupStart = dG; P.cell = dC; P.edge = dE; P.triTag = dT;
         P.geom = dGeom; P.rot = dRot; P.gas = dGas; P.addBase = dAdd; P.count = dCount; P.start = dStart;
         return true;

@@ -32,20 +32,20 @@ constexpr unsigned kFull = 0xffffffffu;
 // path stores absolute FP64; the mixed path stores FP32 offsets from the
 // centre of the particle's cell (widened as centre + offset, stored as the
 // FP32 rounding of position - centre).
-template <typename Real>
+template <typename Real, int kFaces = 0>
 __device__ __forceinline__ void load_position(const DevMesh& M, const PBuf<Real>& B, int i, int cell, PRegs<Real>& p)
 {
     if constexpr (sizeof(Real) == 8) {
         p.x[0] = B.x[0][i]; p.x[1] = B.x[1][i]; p.x[2] = B.x[2][i];
     } else {
-        const double* cc = M.cellCenter + (size_t)cell * 3;
+        const double* cc = cell_centre<kFaces>(M, cell);
         p.x[0] = da(cc[0], (double)B.x[0][i]);
         p.x[1] = da(cc[1], (double)B.x[1][i]);
         p.x[2] = da(cc[2], (double)B.x[2][i]);
     }
 }
 
-template <typename Real>
+template <typename Real, int kFaces = 0>
 __device__ __forceinline__ void store_position(const DevMesh& M, const PBuf<Real>& B, int i, int cell,
                                                const PRegs<Real>& p)
 {
@@ -53,11 +53,60 @@ __device__ __forceinline__ void store_position(const DevMesh& M, const PBuf<Real
         B.x[0][i] = p.x[0]; B.x[1][i] = p.x[1]; B.x[2][i] = p.x[2];
     } else {
         if (cell < 0 || cell >= M.ncell) return;   // removed: the slot is not read again
-        const double* cc = M.cellCenter + (size_t)cell * 3;
+        const double* cc = cell_centre<kFaces>(M, cell);
         B.x[0][i] = (float)ds(p.x[0], cc[0]);
         B.x[1][i] = (float)ds(p.x[1], cc[1]);
         B.x[2][i] = (float)ds(p.x[2], cc[2]);
     }
+}
+
+// The mesh's kind for the kernels that trace: the record stride when the exit
+// search unrolls over it (tetrahedra 4, pyramids and wedges 5, hexahedra 6),
+// else 0. Each kernel holds one kind's search only: with all of them in one
+// kernel it ran slower than unrolling gained (372,500 tetrahedra: the
+// tracing pass 960 -> 1146 us), its code no longer fitting the instruction
+// cache.
+inline int face_kind(const DevMesh& M) { return M.faceStride >= 4 && M.faceStride <= 6 ? M.faceStride : 0; }
+
+// f(integral constant of the kind)
+template <typename F>
+inline void with_face_kind(const DevMesh& M, F&& f)
+{
+    switch (face_kind(M)) {
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        case 5: f(std::integral_constant<int, 5>{}); break;
+        case 6: f(std::integral_constant<int, 6>{}); break;
+        default: f(std::integral_constant<int, 0>{}); break;
+    }
+}
+
+size_t geo_floats(const DevMesh& M)
+{
+    const int f = face_kind(M);
+    return f == 0 ? 0 : f == 6 ? CellGeo<6>::kFloats : CellGeo<4>::kFloats;
+}
+
+template <int kFaces>
+__global__ void pack_geo_kernel(DevMesh M, float4* geo)
+{
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < M.ncell; c += gridDim.x * blockDim.x) {
+        float4* g = geo + (size_t)c * (CellGeo<kFaces>::kFloats / 4);
+        for (int j = 0; j < kFaces; ++j) g[j] = M.planeF[(size_t)c * kFaces + j];
+        double* cc = reinterpret_cast<double*>(g + kFaces);
+        for (int d = 0; d < 3; ++d) cc[d] = M.cellCenter[(size_t)c * 3 + d];
+        float* f = reinterpret_cast<float*>(g + kFaces);
+        f[6] = M.recAux[(size_t)c * kFaces].y;
+        for (int j = 0; j < kFaces; ++j) f[7 + j] = M.recAux[(size_t)c * kFaces + j].x;
+    }
+}
+
+void launch_pack_geo(const DevMesh& M, float4* geo, cudaStream_t s)
+{
+    const int g = (M.ncell + 255) / 256;
+    with_face_kind(M, [&](auto f) {
+        constexpr int F = decltype(f)::value;
+        if constexpr (F > 0) pack_geo_kernel<F><<<g < 2048 ? g : 2048, 256, 0, s>>>(M, geo);
+    });
 }
 
 // ===========================================================================
@@ -176,15 +225,21 @@ __device__ __forceinline__ void sample_inflow_velocity(const double* gas, const 
 // One thread per injected particle; its patch is found by binary search in
 // the exclusive scan of the per-patch counts (slots of one patch are
 // consecutive, so a warp mostly works on one patch).
-template <typename Real>
+template <typename Real, int kFaces>
 __global__ void __launch_bounds__(128) inject_gen_kernel(StepArgs<Real> a)
 {
+    __shared__ ExitHit scanned[128];
     const int istep = a.ctl->istep;
     const int nLive = a.ctl->nLive;
     const int m = a.ctl->nInj;
     const int np = a.P.npatch;
     TraceCounts cnt{};
-    for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < m; slot += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    // whole warps, the lanes past the end with a copy of the last particle
+    // that is not stored (they take part in the warp's traces)
+    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < m; base += gridDim.x * blockDim.x) {
+        const bool mine = base + lane < m;
+        const int slot = min(base + lane, m - 1);
         int lo = 0, hi = np - 1;          // last patch with start <= slot
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -213,9 +268,10 @@ __global__ void __launch_bounds__(128) inject_gen_kernel(StepArgs<Real> a)
         for (int d = 0; d < 3; ++d) pr.x[d] = pos[d];
         for (int d = 0; d < 3; ++d) pr.v[d] = (Real)vel[d];
         pr.ir = (Real)irv;
-        const int out = trace_particle<Real>(a.M, a.C, pr, cell, pedge, ptag, dtleft, rs, istep,
-                                             a.wallTally, cnt, false, nullptr);
-        store_position(a.M, a.A, gi, cell, pr);
+        const int out = trace_particle_warp<Real, kFaces>(mine, a.M, a.C, pr, cell, pedge, ptag, dtleft, rs, istep,
+                                                          a.wallTally, cnt, &scanned[threadIdx.x]);
+        if (!mine) continue;
+        store_position<Real, kFaces>(a.M, a.A, gi, cell, pr);
         a.A.v[0][gi] = pr.v[0]; a.A.v[1][gi] = pr.v[1]; a.A.v[2][gi] = pr.v[2];
         a.A.ir[gi] = pr.ir;
         a.A.cell[gi] = (out >= 0) ? cell : -1;
@@ -233,7 +289,9 @@ void launch_inject(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s
     const int gCount = (a.P.ngroup + 127) / 128;
     inject_count_kernel<<<gCount > 0 ? gCount : 1, 128, 0, s>>>(a.P, a.remInj);
     inject_scan_kernel<<<1, 1024, 0, s>>>(a.P, a.ctl, a.counters);
-    inject_gen_kernel<Real><<<L.smCount * 8, 128, 0, s>>>(a);
+    // one particle a thread at the expected count (a remainder can add one per patch)
+    const int gGen = max(1, min(L.smCount * 8, (a.P.expected + 127) / 128));
+    with_face_kind(a.M, [&](auto f) { inject_gen_kernel<Real, decltype(f)::value><<<gGen, 128, 0, s>>>(a); });
 }
 
 // ===========================================================================
@@ -246,37 +304,50 @@ void launch_inject(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s
 // reads few cells' face records). Most particles stay in their cell for the
 // whole step; where the first exit search settles that (stays_for_the_step)
 // the particle is advanced and stored right there. The others are appended
-// to a work list (warp-aggregated, in the sort's rank array, which is free
-// until the sort), with their state copied to the same positions of the
-// other particle buffer (free until the sort too): the tracing pass then
-// reads its particles in list order instead of gathering them from sparse
-// slots (move 2.18 -> 2.08 ms). (Handing the crossing that search settled
-// to the tracing pass as well was measured slower: 2.37 against 2.17 ms.)
+// to a work list (in the sort's rank array, which is free until the sort),
+// with their state copied to the same positions of the other particle buffer
+// (free until the sort too): the tracing pass then reads its particles in list
+// order instead of gathering them from sparse slots. A block takes its share
+// of the list with one atomic for up to 1,024 particles: with one per warp
+// and 32 particles, the million atomics on one address were the pass (37M
+// particles: 974 us, 634 with one per block). It then waits for the cells'
+// geometry.
 //
 // Tracing pass (move_kernel): the listed particles, traced from their start
 // by trace_step. Warps claim chunks of 128 list entries from a cursor in
 // the step control block (one atomic per chunk), and a lane whose particle
 // has finished writes it back and takes the next particle of the chunk, so
 // the lanes keep doing exit searches instead of waiting for the warp's
-// longest trace. Three resident 256-thread blocks per SM (registers capped
-// at 85): the trace is bound by dependent loads, so occupancy pays more than
-// the few registers it spills to L1.
+// longest trace. A list too short for that gives every warp an equal share
+// instead, down to 8 entries: a warp that refilled its lanes while others had
+// none would only add its rounds to the pass's latency (19,700 particles: 69
+// -> 27 us). Three resident 256-thread blocks per SM (registers capped at 85):
+// the trace is bound by dependent loads, so occupancy pays more than the few
+// registers it spills to L1.
 //
 // Each particle runs the same code with its own random stream (particle
 // index, step), and the stay pass takes exactly the decision the trace's
 // first search takes, so results do not depend on the split, the list
 // order, or which lane or warp traces a particle.
 constexpr int kMoveChunk = 128;
+constexpr int kMoveChunkMin = 8;
 
 // K particles per thread (K x 256 consecutive slots per block and round):
 // the loads of all K are issued before the first decision.
-template <typename Real, int K>
+template <typename Real, int K, int kFaces>
 __global__ void __launch_bounds__(256) move_stay_kernel(StepArgs<Real> a)
 {
+    __shared__ int sCount[2], sBase;
     const int n = a.ctl->nLive;
     const double dt = a.C.dtime;
     const int lane = threadIdx.x & 31;
-    const int tile = K * (int)blockDim.x;
+    int parity = 0;
+    if (threadIdx.x < 2) sCount[threadIdx.x] = 0;
+    __syncthreads();
+    // a step with fewer slots than K a thread takes as many as give every
+    // thread its share, rather than K on few of them
+    const int per = min(K, (n + (int)(gridDim.x * blockDim.x) - 1) / (int)(gridDim.x * blockDim.x));
+    const int tile = per * (int)blockDim.x;
     for (int base = blockIdx.x * tile; base < n; base += gridDim.x * tile) {
         int cell[K];
         Real xs[K][3];
@@ -285,7 +356,7 @@ __global__ void __launch_bounds__(256) move_stay_kernel(StepArgs<Real> a)
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int i = base + k * (int)blockDim.x + (int)threadIdx.x;
-            if (i < n) {
+            if (i < n && k < per) {
                 cell[k] = a.A.cell[i];
                 xs[k][0] = a.A.x[0][i]; xs[k][1] = a.A.x[1][i]; xs[k][2] = a.A.x[2][i];
                 p[k].v[0] = a.A.v[0][i]; p[k].v[1] = a.A.v[1][i]; p[k].v[2] = a.A.v[2][i];
@@ -293,49 +364,65 @@ __global__ void __launch_bounds__(256) move_stay_kernel(StepArgs<Real> a)
                 cell[k] = -1;
             }
         }
+        // the decisions: stayers advanced and stored, the others counted
+        unsigned defer = 0u;
+        int before[K], mine = 0;   // the warp's deferred ones before this lane's of set k
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int i = base + k * (int)blockDim.x + (int)threadIdx.x;
-            bool defer = false;
+            bool d = false;
             if (cell[k] >= 0) {
                 // the position as load_position widens it
                 if constexpr (sizeof(Real) == 8) {
                     p[k].x[0] = xs[k][0]; p[k].x[1] = xs[k][1]; p[k].x[2] = xs[k][2];
                 } else {
-                    const double* cc = a.M.cellCenter + (size_t)cell[k] * 3;
+                    const double* cc = cell_centre<kFaces>(a.M, cell[k]);
                     p[k].x[0] = da(cc[0], (double)xs[k][0]);
                     p[k].x[1] = da(cc[1], (double)xs[k][1]);
                     p[k].x[2] = da(cc[2], (double)xs[k][2]);
                 }
-                if (stays_for_the_step<Real>(a.M, cell[k], p[k], dt)) {
+                if (stays_for_the_step<Real, kFaces>(a.M, cell[k], xs[k], p[k], dt)) {
                     advance(p[k], dt);
-                    store_position(a.M, a.A, i, cell[k], p[k]);
+                    store_position<Real, kFaces>(a.M, a.A, i, cell[k], p[k]);
                 } else {
-                    defer = true;
+                    d = true;
                 }
             }
-            const unsigned m = __ballot_sync(kFull, defer);
-            if (m) {
-                int at = 0;
-                if (lane == 0) at = atomicAdd(&a.ctl->moveList, __popc(m));
-                at = __shfl_sync(kFull, at, 0);
-                if (defer) {
-                    // the entry: the slot, and the particle's state in the
-                    // other buffer (free until the sort) at the same
-                    // position, so the tracing pass reads it in list order
-                    const int j = at + __popc(m & ((1u << lane) - 1u));
-                    a.rank[j] = i;
-                    a.B.cell[j] = cell[k];
-                    a.B.x[0][j] = xs[k][0]; a.B.x[1][j] = xs[k][1]; a.B.x[2][j] = xs[k][2];
-                    a.B.v[0][j] = p[k].v[0]; a.B.v[1][j] = p[k].v[1]; a.B.v[2][j] = p[k].v[2];
-                    a.B.ir[j] = a.A.ir[i];
-                }
-            }
+            const unsigned m = __ballot_sync(kFull, d);
+            before[k] = mine + __popc(m & ((1u << lane) - 1u));
+            mine += __popc(m);
+            if (d) defer |= 1u << k;
+        }
+        // the block's share of the list: one atomic for all of its warps
+        int at = 0;
+        if (lane == 0 && mine) at = atomicAdd(&sCount[parity], mine);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int c = sCount[parity];
+            sBase = c ? atomicAdd(&a.ctl->moveList, c) : 0;
+            sCount[parity ^ 1] = 0;
+        }
+        __syncthreads();
+        at = sBase + __shfl_sync(kFull, at, 0);
+        parity ^= 1;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (!((defer >> k) & 1u)) continue;
+            // the entry: the slot, and the particle's state in the other
+            // buffer (free until the sort) at the same position, so the
+            // tracing pass reads it in list order
+            const int i = base + k * (int)blockDim.x + (int)threadIdx.x;
+            const int j = at + before[k];
+            a.rank[j] = i;
+            a.B.cell[j] = cell[k];
+            a.B.x[0][j] = xs[k][0]; a.B.x[1][j] = xs[k][1]; a.B.x[2][j] = xs[k][2];
+            a.B.v[0][j] = p[k].v[0]; a.B.v[1][j] = p[k].v[1]; a.B.v[2][j] = p[k].v[2];
+            a.B.ir[j] = a.A.ir[i];
         }
     }
 }
 
-template <typename Real>
+template <typename Real, int kFaces>
 __global__ void __launch_bounds__(256, 3) move_kernel(StepArgs<Real> a)
 {
     const int istep = a.ctl->istep;
@@ -345,6 +432,8 @@ __global__ void __launch_bounds__(256, 3) move_kernel(StepArgs<Real> a)
     const unsigned lower = (1u << lane) - 1u;
     TraceCounts cnt{};
     const double dt0 = a.C.dtime;
+    const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+    const int chunk = max(kMoveChunkMin, min(kMoveChunk, (n + warps - 1) / warps));
     int chunkNext = 0, chunkEnd = 0;   // this warp's chunk (warp-uniform)
     bool exhausted = false;            // warp-uniform
     int i = -1;                        // this lane's particle
@@ -362,14 +451,14 @@ __global__ void __launch_bounds__(256, 3) move_kernel(StepArgs<Real> a)
         while (want && !exhausted) {
             if (chunkNext >= chunkEnd) {
                 int base = 0;
-                if (lane == 0) base = atomicAdd(&a.ctl->moveCursor, kMoveChunk);
+                if (lane == 0) base = atomicAdd(&a.ctl->moveCursor, chunk);
                 base = __shfl_sync(kFull, base, 0);
                 if (base >= n) {
                     exhausted = true;
                     break;
                 }
                 chunkNext = base;
-                chunkEnd = min(base + kMoveChunk, n);
+                chunkEnd = min(base + chunk, n);
             }
             const int take = min(chunkEnd - chunkNext, __popc(want));
             const bool mine = ((want >> lane) & 1u) && __popc(want & lower) < take;
@@ -378,7 +467,7 @@ __global__ void __launch_bounds__(256, 3) move_kernel(StepArgs<Real> a)
                 const int j = chunkNext + __popc(want & lower);
                 i = list[j];
                 cell = a.B.cell[j];
-                load_position(a.M, a.B, j, cell, p);
+                load_position<Real, kFaces>(a.M, a.B, j, cell, p);
                 p.v[0] = a.B.v[0][j]; p.v[1] = a.B.v[1][j]; p.v[2] = a.B.v[2][j];
                 p.ir = a.B.ir[j];
                 if constexpr (sizeof(Real) == 4) rs.init((uint32_t)i, (uint32_t)istep, kPurposeWall);
@@ -392,9 +481,10 @@ __global__ void __launch_bounds__(256, 3) move_kernel(StepArgs<Real> a)
         }
         const bool active = i >= 0;
         if (!__any_sync(kFull, active)) break;
-        if (active && trace_step<Real, Rng>(a.M, a.C, p, cell, dtleft, st, rs, istep, a.wallTally, cnt, false, nullptr)) {
+        if (active && trace_step<Real, Rng, kFaces, false>(a.M, a.C, p, cell, dtleft, st, rs, istep, a.wallTally, cnt,
+                                                           false, nullptr)) {
             if (st.ifout >= 0) {
-                store_position(a.M, a.A, i, cell, p);
+                store_position<Real, kFaces>(a.M, a.A, i, cell, p);
                 if (cnt.wall != wallBefore) {
                     a.A.v[0][i] = p.v[0]; a.A.v[1][i] = p.v[1]; a.A.v[2][i] = p.v[2];
                     a.A.ir[i] = p.ir;
@@ -409,14 +499,36 @@ __global__ void __launch_bounds__(256, 3) move_kernel(StepArgs<Real> a)
     flush_counts(a.counters, cnt);
 }
 
-// resident blocks per SM of the stay pass (1, 2, 4 particles per thread),
-// set by prepare_kernels
+// resident blocks per SM of the stay pass (1, 2, 4 particles per thread) by
+// kind, set by prepare_kernels
 template <typename Real>
 struct StayOcc {
-    static int blocks[3];
+    static int blocks[7][3];
 };
 template <typename Real>
-int StayOcc<Real>::blocks[3] = {4, 4, 4};
+int StayOcc<Real>::blocks[7][3];
+
+template <typename Real>
+cudaError_t prepare_move()
+{
+    cudaError_t e = cudaSuccess;
+    auto blocks = [&](const void* k, int threads, int& out) {
+        int nb = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, 0);
+        out = nb > 0 ? nb : 1;
+    };
+    auto kind = [&](auto f) {
+        constexpr int F = decltype(f)::value;
+        blocks((const void*)move_stay_kernel<Real, 1, F>, 256, StayOcc<Real>::blocks[F][0]);
+        blocks((const void*)move_stay_kernel<Real, 2, F>, 256, StayOcc<Real>::blocks[F][1]);
+        blocks((const void*)move_stay_kernel<Real, 4, F>, 256, StayOcc<Real>::blocks[F][2]);
+    };
+    kind(std::integral_constant<int, 0>{});
+    kind(std::integral_constant<int, 4>{});
+    kind(std::integral_constant<int, 5>{});
+    kind(std::integral_constant<int, 6>{});
+    return e;
+}
 
 template <typename Real>
 void launch_move(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s)
@@ -424,15 +536,16 @@ void launch_move(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s)
     static_assert(offsetof(StepCtl, moveList) == offsetof(StepCtl, moveCursor) + sizeof(int),
                   "the move's cursor and list count are reset together");
     cudaMemsetAsync(&a.ctl->moveCursor, 0, 2 * sizeof(int), s);
-    // one wave: every block resident (the blocks split the slots evenly, so
-    // a second, partial wave would run at a fraction of the occupancy)
-    if (L.stayPerThread == 4)
-        move_stay_kernel<Real, 4><<<L.smCount * StayOcc<Real>::blocks[2], 256, 0, s>>>(a);
-    else if (L.stayPerThread == 2)
-        move_stay_kernel<Real, 2><<<L.smCount * StayOcc<Real>::blocks[1], 256, 0, s>>>(a);
-    else
-        move_stay_kernel<Real, 1><<<L.smCount * StayOcc<Real>::blocks[0], 256, 0, s>>>(a);
-    move_kernel<Real><<<L.smCount * L.moveBlocksPerSm, L.moveThreads, 0, s>>>(a);
+    with_face_kind(a.M, [&](auto f) {
+        constexpr int F = decltype(f)::value;
+        // one wave: every block resident (the blocks split the slots evenly,
+        // so a second, partial wave would run at a fraction of the occupancy)
+        const int* occ = StayOcc<Real>::blocks[F];
+        if (L.stayPerThread == 4) move_stay_kernel<Real, 4, F><<<L.smCount * occ[2], 256, 0, s>>>(a);
+        else if (L.stayPerThread == 2) move_stay_kernel<Real, 2, F><<<L.smCount * occ[1], 256, 0, s>>>(a);
+        else move_stay_kernel<Real, 1, F><<<L.smCount * occ[0], 256, 0, s>>>(a);
+        move_kernel<Real, F><<<L.smCount * L.moveBlocksPerSm, L.moveThreads, 0, s>>>(a);
+    });
 }
 
 // advance the step counter on the device (batched steps, where the graph
@@ -1659,14 +1772,7 @@ cudaError_t prepare_kernels()
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, collide_kernel<Real>, kCellWarps * 32, cellBytes);
     if (e != cudaSuccess) return e;
     CellOcc<Real>::blocks = nb > 0 ? nb : 1;
-    const void* stay[3] = {(const void*)move_stay_kernel<Real, 1>, (const void*)move_stay_kernel<Real, 2>,
-                           (const void*)move_stay_kernel<Real, 4>};
-    for (int k = 0; k < 3; ++k) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stay[k], 256, 0);
-        if (e != cudaSuccess) return e;
-        StayOcc<Real>::blocks[k] = nb > 0 ? nb : 1;
-    }
-    return cudaSuccess;
+    return prepare_move<Real>();
 }
 
 template <typename Real>

@@ -28,6 +28,7 @@ struct StepCtl {
 
 struct DevPatches {
     int npatch, ngroup;
+    int expected;              // particles a step injects, at most about
     const int* groupStart;     // [ngroup+1] into patch arrays (patches grouped by cell)
     const int* cell;           // [npatch]
     const int* edge;           // [npatch]
@@ -153,6 +154,10 @@ void launch_upload_check(const int* cell, int n, int ncell, int* flags, int* sta
 // out[i] = (float)(in[i] - center[cell[i] * 3 + comp]) for comp < 3, else (float)in[i]
 void launch_upload_convert(const double* in, const int* cell, const double* center, int comp, float* out, int n,
                            cudaStream_t s);
+// The searches' blocks (CellGeo) from the mesh's arrays: floats per cell, 0
+// where the mesh has no such blocks, and their packing.
+size_t geo_floats(const DevMesh& M);
+void launch_pack_geo(const DevMesh& M, float4* geo, cudaStream_t s);
 template <typename Real> cudaError_t prepare_kernels();
 void launch_macro(const DevMesh& M, const DevConsts& C, const double* acc, int set, double count,
                   double* out, int ncell, cudaStream_t s);
