@@ -840,9 +840,9 @@ struct Engine {
             !alloc(windowValid, (size_t)ncell) || !alloc(wallTally, (size_t)std::max(nwall, 1) * 6) ||
             !alloc(countSlot, (size_t)ncell * kSlots) || !alloc(scanPartial, kScanBlocks) ||
             !alloc(start[0], (size_t)ncell + 1) || !alloc(start[1], (size_t)ncell + 1) || !alloc(ctl, 1) ||
-            !alloc(counters, C_COUNT) || !alloc(cellList, (size_t)ncell * 2) || !alloc(cellWork, 8) ||
+            !alloc(counters, C_COUNT) || !alloc(cellList, (size_t)ncell * 2) || !alloc(cellWork, 16) ||
             !alloc(cellPairs, (size_t)ncell) || !alloc(cellCons, (size_t)ncell) ||
-            !alloc(cellItem, (size_t)ncell) || !alloc(cellItemC, (size_t)ncell) ||
+            !alloc(cellItem, (size_t)ncell * 2) || !alloc(cellItemC, (size_t)ncell * 2) ||
             !alloc(errorWord, 1) || !alloc(uploadFlag, 1))
             return false;
         if (params.keep_step_moments && !alloc(stepMom, (size_t)ncell * 18)) return false;

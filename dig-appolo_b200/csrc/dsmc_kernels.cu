@@ -1025,24 +1025,40 @@ struct PState {
 // pair, the post-collision state (pair_execute). pair_execute recomputes the
 // relative velocity from the same stored velocities, so the halves give the
 // bits of the one-piece test-and-collide. w2, w3: words 2 and 3 of the
-// pair's block 0; cr: the relative speed, for the cell's crmax. The FP64
+// pair's block 0; speed: for the cell's crmax, the relative speed in FP32 and
+// its square in FP64 (largest_speed takes the root of the largest). The FP64
 // branch rounds each operation on its own in the reference's evaluation
 // order; the FP32 branch lets the compiler fuse.
 template <typename Real>
 __device__ __forceinline__ bool pair_accept(const PState<Real>& p, const PState<Real>& q, uint32_t w2, uint32_t w3,
-                                            const DevConsts& C, double consCrm, Real crm0, bool splitSum, Real& cr)
+                                            const DevConsts& C, double consCrm, Real crm0, bool splitSum, Real& speed)
 {
     if constexpr (sizeof(Real) == 8) {
         const double vr0 = ds(p.x, q.x), vr1 = ds(p.y, q.y), vr2 = ds(p.z, q.z);
-        cr = sqrt(da(da(dm(vr0, vr0), dm(vr1, vr1)), dm(vr2, vr2)));
-        const double accept = dd(collision_diameter(dm(cr, C.vrms), C.cdPrefactor, C.eta), consCrm);
-        return unit64(w2, w3) < accept;
+        const double cr2 = da(da(dm(vr0, vr0), dm(vr1, vr1)), dm(vr2, vr2));
+        speed = cr2;
+        const double u = unit64(w2, w3);
+        // The acceptance is (cr / crmax)^(1 - 2 eta). In FP32 it comes out
+        // within 3e-6 of itself for ratios of 2^-60 to 2^60 (the logarithm's
+        // error times its exponent); a variate further than 2^-13 of it away
+        // is settled, and only the others (1 in 10^4) need the square root,
+        // the power and the division of the FP64 test.
+        const float c0 = (float)crm0;
+        const float r = __fdividef((float)cr2, c0 * c0);
+        if (r > 0x1p-60f && r < 0x1p60f) {
+            const float est = exp2f(0.5f * C.vhsExpF * __log2f(r)), uf = (float)u;
+            if (uf < est * (1.0f - 0x1p-13f)) return true;
+            if (uf > est * (1.0f + 0x1p-13f)) return false;
+        }
+        const double accept = dd(collision_diameter(dm(sqrt(cr2), C.vrms), C.cdPrefactor, C.eta), consCrm);
+        return u < accept;
     } else {
         const float vr0 = p.x - q.x, vr1 = p.y - q.y, vr2 = p.z - q.z;
         // the squares added in one rounding each; in cells whose pairs ran
         // in place or alone (splitSum) the last one is rounded on its own
         const float xy = fmaf(vr0, vr0, __fmul_rn(vr1, vr1));
-        cr = psqrt(splitSum ? __fadd_rn(xy, __fmul_rn(vr2, vr2)) : fmaf(vr2, vr2, xy));
+        const float cr = psqrt(splitSum ? __fadd_rn(xy, __fmul_rn(vr2, vr2)) : fmaf(vr2, vr2, xy));
+        speed = cr;
         // ratio of the VHS sigma*c at cr and at crmax: (cr/crmax)^(1-2 eta)
         const float accept = exp2f(C.vhsExpF * __log2f(__fdividef(cr, crm0)));
         return unit32(w2) < accept;
@@ -1075,7 +1091,8 @@ __device__ __forceinline__ void pair_execute_fp64(PState<double>& p, PState<doub
     const double cosChi = ds(dm(2.0, pow(rChi, C.invAlpha)), 1.0);
     const double sinChi = sqrt(ds(1.0, dm(cosChi, cosChi)));
     const double ang = dm(6.283185307179586, th);   // 2 pi th
-    const double sth = sin(ang), cth = cos(ang);
+    double sth, cth;
+    sincos(ang, &sth, &cth);
     const double vrp = sqrt(da(dm(vr1, vr1), dm(vr2, vr2)));
     const double scale = dd(postVr, cr > 1.0e-300 ? cr : 1.0e-300);
     const double vrpc = vrp > 1.0e-300 ? vrp : 1.0e-300;
@@ -1140,28 +1157,29 @@ __device__ __forceinline__ void pair_execute_fp32(PState<float>& p, PState<float
 }
 
 // One candidate pair (j of cell c) on the two particles' states: tested and,
-// when accepted, carried out. The draws of the second half do not depend on
-// the test, so in FP32 they are made beside it (the lanes of a warp that
-// reject would wait for those that accept in any case). Returns whether the
-// pair was accepted; crmLocal takes the relative speed if it is larger.
+// when accepted, carried out. Returns whether it was accepted; crmLocal takes
+// pair_accept's speed if it is larger.
 template <typename Real>
 __device__ __forceinline__ bool pair_collide(PState<Real>& p, PState<Real>& q, int c, int istep, int j, uint32_t w2,
                                              uint32_t w3, const DevConsts& C, double consCrm, Real crm0, bool splitSum,
                                              Real& crmLocal)
 {
-    PairDraw d;
-    d.c = (uint32_t)c; d.istep = (uint32_t)istep; d.purpose = kPurposeCollide | ((uint32_t)j << 4);
-    U4 b1;
-    if constexpr (sizeof(Real) == 4) b1 = d.block(1, C);
-    Real cr;
-    const bool acc = pair_accept<Real>(p, q, w2, w3, C, consCrm, crm0, splitSum, cr);
-    if (cr > crmLocal) crmLocal = cr;
+    Real speed;
+    const bool acc = pair_accept<Real>(p, q, w2, w3, C, consCrm, crm0, splitSum, speed);
+    if (speed > crmLocal) crmLocal = speed;
     if (acc) {
+        PairDraw d;
+        d.c = (uint32_t)c; d.istep = (uint32_t)istep; d.purpose = kPurposeCollide | ((uint32_t)j << 4);
         if constexpr (sizeof(Real) == 8) pair_execute_fp64(p, q, d, C);
-        else pair_execute_fp32(p, q, b1, w3, C);
+        else pair_execute_fp32(p, q, d.block(1, C), w3, C);
     }
     return acc;
 }
+
+// The largest relative speed from the largest value pair_accept gave (the
+// square root, rounded as it is, keeps the order).
+__device__ __forceinline__ double largest_speed(double m) { return sqrt(m); }
+__device__ __forceinline__ double largest_speed(float m) { return (double)m; }
 
 // Candidate pair count of a cell from the majorant, with the carried
 // remainder (collisionDSMC, src/ProcessDSMC.cpp:2631-2645), in the
@@ -1209,7 +1227,20 @@ __device__ void collide_cell_serial(Real* const (&v)[4], int stride, int n, int 
             ++collOut;
         }
     }
-    if ((double)crmLocal > crm0) a.crmax[c] = (double)crmLocal;
+    const double crm = largest_speed(crmLocal);
+    if (crm > crm0) a.crmax[c] = crm;
+}
+
+// the largest of a warp's values
+template <typename Real>
+__device__ __forceinline__ Real warp_max(Real m)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const Real y = __shfl_xor_sync(kFull, m, o);
+        m = y > m ? y : m;
+    }
+    return m;
 }
 
 // NTC collisions of one cell by one warp, in place in the particle buffer,
@@ -1269,25 +1300,20 @@ __device__ void collide_cell_in_place(const PBuf<Real>& buf, int s0, int n, int 
         }
         __syncwarp();
     }
-    Real m = crmLocal;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const Real y = __shfl_xor_sync(kFull, m, o);
-        m = y > m ? y : m;
-    }
-    if (lane == 0 && (double)m > crm0) a.crmax[c] = (double)m;
+    const double m = largest_speed(warp_max(crmLocal));
+    if (lane == 0 && m > crm0) a.crmax[c] = m;
     for (int k = lane; k < n; k += 32) claim[k] = c;
     __syncwarp();
 }
 
 // The collision pass over the sorted buffer (collisionDSMC,
 // src/ProcessDSMC.cpp:2621-2665). Cells are classed first (classify_kernel):
-// - small cells (at most kSmallMax particles): 32 at a time per warp, lane
-//   l owning one cell and running its pairs alone, with the particles'
+// - small cells (at most kSmallMax particles and kSmallPairs pairs): 32 at a
+//   time per warp, lane l owning one cell and running its pairs alone, with the particles'
 //   velocities and internal energies in shared memory at slot k * 32 + l
 //   (lane l's slots sit in bank l, so the lanes never conflict);
 // - large cells: two at a time per warp, staged in shared memory
-//   (collide_kernel);
+//   (collide_kernel), those of the most rounds first;
 // - big cells (more particles than a warp's arena, or more pairs than
 //   kBigPairs) and giants (more pairs than kGiantPairs, handed out first):
 //   one at a time by a block of 512 threads (collide_big_kernel), beside the
@@ -1300,7 +1326,8 @@ __device__ void collide_cell_in_place(const PBuf<Real>& buf, int s0, int n, int 
 // chain. With every cell run by one warp, 32 pairs a round at most, the few
 // compressed cells of a capsule (2,000 particles, 30,000-60,000 pairs) were
 // the whole pass. A block runs up to 512 pairs a round (n / 4 (1 - e^(-2048 / n))
-// of them go), in a tenth of the rounds.
+// of them go), in a tenth of the rounds. Next longest were cells of up to 16
+// particles with up to 900 pairs, one lane running one after another.
 constexpr int kCellWarps = 2;                 // warps per block of collide_kernel
 constexpr int kSmallMax = 16;
 constexpr int kArena = 512;                   // staged particles per warp
@@ -1308,6 +1335,8 @@ static_assert(32 * kSmallMax <= kArena, "small-cell slots must fit in the arena"
 constexpr int kBigThreads = 512;
 constexpr int kBigArena = 4096;               // staged particles per block of collide_big_kernel
 constexpr int kBigPairs = 1024;
+constexpr int kBigLeast = 128;                // fewer particles give a block no more pairs a round than a warp
+constexpr int kSmallPairs = 32;
 constexpr int kGiantPairs = 8192;
 
 // shared memory of `slots` staged particles: their states and claims
@@ -1390,11 +1419,20 @@ __device__ __forceinline__ void unstage_cell(const PBuf<Real>& buf, const Arena<
     }
 }
 
-// cellWork: [0] large count, [1] small count, [2] big count, [3] giant count,
-//           [4] next large item, [5] next small item, [6] next giant or big
+// cellWork: [0..2] large counts by their rounds (more than kManyRounds, more
+//           than kSomeRounds, the rest), [3] small count, [4] big count, [5] giant
+//           count, [6] next large item, [7] next small, [8] next giant or big
 // cellList: small cells from the front of [0, ncell), big cells from its
 //           back, giants from the front of [ncell, 2 ncell)
-// cellItem: large cells
+// cellItem: large cells, of many rounds from the front of [0, ncell), of some
+//           from its back, the rest from the front of [ncell, 2 ncell); handed
+//           out in this order, so that the longest chains start first
+constexpr int kWorkWords = 16;
+constexpr int kManyRounds = 40, kSomeRounds = 12;
+__device__ __forceinline__ int large_slot(int it, int n0, int n1, int ncell)
+{
+    return it < n0 ? it : it < n0 + n1 ? ncell - 1 - (it - n0) : ncell + (it - n0 - n1);
+}
 template <typename Real>
 __global__ void classify_kernel(StepArgs<Real> a)
 {
@@ -1420,12 +1458,15 @@ __global__ void classify_kernel(StepArgs<Real> a)
         // nothing collides in a cell without pairs: it goes on no list
         int cls = -1;
         if (n > 1 && np > 0 && consCrm > 0.0) {
-            if (n <= kSmallMax) cls = 1;
-            else if (np > kGiantPairs) cls = 3;
-            else cls = n > kArena || np > kBigPairs ? 2 : 0;
+            // a round runs about 13 pairs of a cell, n / 4 of one with few particles
+            const int rounds = np / min(13, max(1, n >> 2));
+            if (n <= kSmallMax && np <= kSmallPairs) cls = 3;
+            else if (np > kGiantPairs && n > kBigLeast) cls = 5;
+            else if (n > kArena || (np > kBigPairs && n > kBigLeast)) cls = 4;
+            else cls = rounds > kManyRounds ? 0 : rounds > kSomeRounds ? 1 : 2;
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < 6; ++k) {
             const unsigned m = __ballot_sync(kFull, cls == k);
             if (!m) continue;
             const int leader = __ffs(m) - 1;
@@ -1434,11 +1475,12 @@ __global__ void classify_kernel(StepArgs<Real> a)
             b = __shfl_sync(kFull, b, leader);
             if (cls == k) {
                 const int pos = b + __popc(m & ((1u << lane) - 1u));
-                if (k == 0) {
-                    a.cellItem[pos] = make_int4(c, s0, n, np);
-                    a.cellItemC[pos] = make_double2(consCrm, crm0);
+                if (k < 3) {
+                    const int slot = k == 0 ? pos : k == 1 ? ncell - 1 - pos : ncell + pos;
+                    a.cellItem[slot] = make_int4(c, s0, n, np);
+                    a.cellItemC[slot] = make_double2(consCrm, crm0);
                 } else {
-                    a.cellList[k == 1 ? pos : k == 2 ? ncell - 1 - pos : ncell + pos] = c;
+                    a.cellList[k == 3 ? pos : k == 4 ? ncell - 1 - pos : ncell + pos] = c;
                 }
             }
         }
@@ -1469,18 +1511,6 @@ __device__ __forceinline__ void copy_cell(const PBuf<Real>& buf, int s0, int n, 
         }
 }
 
-// the largest of a warp's values
-template <typename Real>
-__device__ __forceinline__ Real warp_max(Real m)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const Real y = __shfl_xor_sync(kFull, m, o);
-        m = y > m ? y : m;
-    }
-    return m;
-}
-
 // Collisions of staged large cells, two cells per warp at a time, both in
 // the warp's arena: channel 0's cell at slots [0, n0), channel 1's at
 // [kArena - n1, kArena); a cell that does not fit beside the other channel's
@@ -1500,8 +1530,8 @@ __device__ __forceinline__ Real warp_max(Real m)
 // some 13 to 20 go a round, and of 16 about 13; each phase then runs once a
 // round for both cells.
 template <typename Real>
-__device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf, const Arena<Real>& A, int nItems,
-                                  int istep, uint32_t& colls)
+__device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf, const Arena<Real>& A, int n0, int n1,
+                                  int nItems, int istep, uint32_t& colls)
 {
     constexpr int N = kArena;
     const int lane = threadIdx.x & 31;
@@ -1518,7 +1548,31 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
     // handed out in increasing order and the loop runs until it sees one
     // past the end, so an index taken ahead is always used.
     int ahead = 0;
-    if (lane == 0) ahead = atomicAdd(a.cellWork + 4, 1);
+    if (lane == 0) ahead = atomicAdd(a.cellWork + 6, 1);
+    // the next pairs, in increasing order, to the lanes that ask for one (all
+    // lanes call it): of the half's own channel, or of the other when that
+    // has none left; j = -1 for a lane that gets none
+    auto hand_out = [&](bool ask) {
+        const bool left0 = cc[0] >= 0 && cnext[0] < cnp[0], left1 = cc[1] >= 0 && cnext[1] < cnp[1];
+        const int want = !ask ? -1 : lane < 16 ? (left0 ? 0 : left1 ? 1 : -1) : (left1 ? 1 : left0 ? 0 : -1);
+        const unsigned m0 = __ballot_sync(kFull, want == 0), m1 = __ballot_sync(kFull, want == 1);
+        if (ask) {
+            j = -1;
+            const int jj = (want > 0 ? cnext[1] : cnext[0]) + __popc((want > 0 ? m1 : m0) & below);
+            if (want >= 0 && jj < (want ? cnp[1] : cnp[0])) {
+                j = jj;
+                ch = want;
+                const int base = want ? cbase[1] : cbase[0];
+                const PairDraw d = pair_draw(want ? cc[1] : cc[0], istep, jj, want ? cn[1] : cn[0], a.C, k1, k2);
+                k1 += base;
+                k2 += base;
+                w2 = d.b0.z;
+                w3 = d.b0.w;
+            }
+        }
+        cnext[0] = min(cnp[0], cnext[0] + __popc(m0));
+        cnext[1] = min(cnp[1], cnext[1] + __popc(m1));
+    };
     for (;;) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -1526,15 +1580,16 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
                 int it = held;
                 if (it < 0) {
                     it = __shfl_sync(kFull, ahead, 0);
-                    if (lane == 0 && it < nItems) ahead = atomicAdd(a.cellWork + 4, 1);
+                    if (lane == 0 && it < nItems) ahead = atomicAdd(a.cellWork + 6, 1);
                 }
                 held = -1;
                 if (it >= nItems) {
                     more = false;
                     break;
                 }
-                const int4 rec = a.cellItem[it];
-                const double2 rc = a.cellItemC[it];
+                const int slot = large_slot(it, n0, n1, a.M.ncell);
+                const int4 rec = a.cellItem[slot];
+                const double2 rc = a.cellItemC[slot];
                 const int n = rec.z;
                 if (n > N) {   // never reached (classify lists no such cell): flag rather than overflow the arena
                     if (lane == 0) atomicOr(a.errorWord, kErrStageCell);
@@ -1552,25 +1607,7 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
             }
         }
         if (cc[0] < 0 && cc[1] < 0) break;
-        // hand out the next pairs to idle lanes
-        const bool left0 = cc[0] >= 0 && cnext[0] < cnp[0], left1 = cc[1] >= 0 && cnext[1] < cnp[1];
-        const int want = j >= 0 ? -1 : lane < 16 ? (left0 ? 0 : left1 ? 1 : -1) : (left1 ? 1 : left0 ? 0 : -1);
-        const unsigned m0 = __ballot_sync(kFull, want == 0), m1 = __ballot_sync(kFull, want == 1);
-        if (want >= 0) {
-            const int jj = (want ? cnext[1] : cnext[0]) + __popc((want ? m1 : m0) & below);
-            if (jj < (want ? cnp[1] : cnp[0])) {
-                j = jj;
-                ch = want;
-                const int base = want ? cbase[1] : cbase[0];
-                const PairDraw d = pair_draw(want ? cc[1] : cc[0], istep, jj, want ? cn[1] : cn[0], a.C, k1, k2);
-                k1 += base;
-                k2 += base;
-                w2 = d.b0.z;
-                w3 = d.b0.w;
-            }
-        }
-        cnext[0] = min(cnp[0], cnext[0] + __popc(m0));
-        cnext[1] = min(cnp[1], cnext[1] + __popc(m1));
+        hand_out(j < 0);
         // claim both particles with the pair index; the lowest claim goes
         if (j >= 0) {
             atomicMin(&A.claim[k1], j);
@@ -1582,8 +1619,9 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
         if (go) {
             PState<Real> p = A.get(k1), q = A.get(k2);
             Real& crm = ch ? crmL[1] : crmL[0];
+            const int n = ch ? cn[1] : cn[0];
             if (pair_collide<Real>(p, q, ch ? cc[1] : cc[0], istep, j, w2, w3, a.C, ch ? ccons[1] : ccons[0],
-                                   (Real)(ch ? ccrm[1] : ccrm[0]), false, crm)) {
+                                   (Real)(ch ? ccrm[1] : ccrm[0]), n <= kSmallMax, crm)) {
                 A.put(k1, p);
                 A.put(k2, q);
                 ++colls;
@@ -1597,8 +1635,8 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             if (cc[h] < 0 || cnext[h] < cnp[h] || __ballot_sync(kFull, j >= 0 && ch == h) != 0u) continue;
-            const Real m = warp_max(crmL[h]);
-            if (lane == 0 && (double)m > ccrm[h]) a.crmax[cc[h]] = (double)m;
+            const double m = largest_speed(warp_max(crmL[h]));
+            if (lane == 0 && m > ccrm[h]) a.crmax[cc[h]] = m;
             unstage_cell(buf, A, cs0[h], cn[h], cbase[h], lane, 32);
             __syncwarp();
             cc[h] = -1;
@@ -1619,8 +1657,8 @@ __global__ void __launch_bounds__(kCellWarps * 32, sizeof(Real) == 4 ? 10 : 6) c
     const PBuf<Real> buf = a.A;
     uint32_t colls = 0;
 
-    const int nLarge = a.cellWork[0], nSmall = a.cellWork[1];
-    if (nLarge > 0) collide_two_cells<Real>(a, buf, Arena<Real>(wsm, kArena), nLarge, istep, colls);
+    const int n0 = a.cellWork[0], n1 = a.cellWork[1], nLarge = n0 + n1 + a.cellWork[2], nSmall = a.cellWork[3];
+    if (nLarge > 0) collide_two_cells<Real>(a, buf, Arena<Real>(wsm, kArena), n0, n1, nLarge, istep, colls);
 
     // ---- small cells, 32 per warp, one lane each
     constexpr int kSmallSlots = 32 * kSmallMax;
@@ -1629,7 +1667,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, sizeof(Real) == 4 ? 10 : 6) c
     const int* start = a.startA;
     while (nSmall > 0) {
         int g = 0;
-        if (lane == 0) g = atomicAdd(a.cellWork + 5, 32);
+        if (lane == 0) g = atomicAdd(a.cellWork + 7, 32);
         g = __shfl_sync(kFull, g, 0);
         if (g >= nSmall) break;
         const bool mine = g + lane < nSmall;
@@ -1673,14 +1711,14 @@ __global__ void __launch_bounds__(kBigThreads, 1) collide_big_kernel(StepArgs<Re
     const unsigned below = (1u << lane) - 1u;
     const Arena<Real> A(cellSmem, kBigArena);
     const int istep = a.ctl->istep, ncell = a.M.ncell;
-    const int nBig = a.cellWork[2], nGiant = a.cellWork[3];
+    const int nBig = a.cellWork[4], nGiant = a.cellWork[5];
     const PBuf<Real> buf = a.A;
     uint32_t colls = 0;
     if (nBig + nGiant > 0)
         for (;;) {
             __syncthreads();   // the last cell's values have been read
             if (tid == 0) {
-                sItem = atomicAdd(a.cellWork + 6, 1);
+                sItem = atomicAdd(a.cellWork + 8, 1);
                 sNext = 0;
                 sCrm = 0ull;
             }
@@ -1698,26 +1736,31 @@ __global__ void __launch_bounds__(kBigThreads, 1) collide_big_kernel(StepArgs<Re
             __syncthreads();
             const Real crm0r = (Real)crm0;
             Real crmLocal = (Real)0;
+            // threads with pairs: more than n / 2 at once mostly wait for each
+            // other and take issue slots from those that go
+            const bool works = tid < min(kBigThreads, max(64, (n >> 1) & ~31));
             int j = -1, k1 = 0, k2 = 0;
             uint32_t w2 = 0u, w3 = 0u;
-            bool left = true;   // pairs may be left to hand out
-            for (;;) {
-                if (left) {     // the same in every lane of a warp
-                    const unsigned idle = __ballot_sync(kFull, j < 0);
-                    if (idle) {
-                        int first = 0;
-                        if (lane == 0) first = atomicAdd(&sNext, __popc(idle));
-                        first = __shfl_sync(kFull, first, 0);
-                        const int jj = first + __popc(idle & below);
-                        if (j < 0 && jj < np) {
-                            j = jj;
-                            const PairDraw d = pair_draw(c, istep, j, n, a.C, k1, k2);
-                            w2 = d.b0.z;
-                            w3 = d.b0.w;
-                        }
-                        left = first < np;
-                    }
+            bool left = works;  // pairs may be left to hand out (the same in every lane of a warp)
+            // the next pairs to the lanes of this warp that ask for one
+            auto hand_out = [&](bool ask) {
+                const unsigned m = __ballot_sync(kFull, ask);
+                if (ask) j = -1;
+                if (!left || !m) return;
+                int first = 0;
+                if (lane == 0) first = atomicAdd(&sNext, __popc(m));
+                first = __shfl_sync(kFull, first, 0);
+                const int jj = first + __popc(m & below);
+                if (ask && jj < np) {
+                    j = jj;
+                    const PairDraw d = pair_draw(c, istep, j, n, a.C, k1, k2);
+                    w2 = d.b0.z;
+                    w3 = d.b0.w;
                 }
+                left = first < np;
+            };
+            hand_out(works);
+            for (;;) {
                 if (j >= 0) {
                     atomicMin(&A.claim[k1], j);
                     atomicMin(&A.claim[k2], j);
@@ -1725,24 +1768,26 @@ __global__ void __launch_bounds__(kBigThreads, 1) collide_big_kernel(StepArgs<Re
                 __syncthreads();
                 const bool go = j >= 0 && A.claim[k1] == j && A.claim[k2] == j;
                 __syncthreads();
+                const int jNow = j, k1Now = k1, k2Now = k2;
+                const uint32_t w2Now = w2, w3Now = w3;
+                hand_out(go);   // drawn beside this round's collisions, claimed in the next
                 if (go) {
-                    PState<Real> p = A.get(k1), q = A.get(k2);
-                    if (pair_collide<Real>(p, q, c, istep, j, w2, w3, a.C, consCrm, crm0r, n > kArena,
+                    PState<Real> p = A.get(k1Now), q = A.get(k2Now);
+                    if (pair_collide<Real>(p, q, c, istep, jNow, w2Now, w3Now, a.C, consCrm, crm0r, n > kArena,
                                            crmLocal)) {
-                        A.put(k1, p);
-                        A.put(k2, q);
+                        A.put(k1Now, p);
+                        A.put(k2Now, q);
                         ++colls;
                     }
-                    A.claim[k1] = INT_MAX;
-                    A.claim[k2] = INT_MAX;
-                    j = -1;
+                    A.claim[k1Now] = INT_MAX;
+                    A.claim[k2Now] = INT_MAX;
                 }
-                if (!__syncthreads_or(left || j >= 0)) break;
+                if (!__syncthreads_or(j >= 0)) break;
             }
             // the largest relative speed tested (a double's order is that of
             // its bits when positive)
-            const Real m = warp_max(crmLocal);
-            if (lane == 0 && (double)m > crm0) atomicMax(&sCrm, (unsigned long long)__double_as_longlong((double)m));
+            const double m = largest_speed(warp_max(crmLocal));
+            if (lane == 0 && m > crm0) atomicMax(&sCrm, (unsigned long long)__double_as_longlong(m));
             unstage_cell(buf, A, s0, n, 0, tid, kBigThreads);
             __syncthreads();
             if (tid == 0 && sCrm) a.crmax[c] = __longlong_as_double((long long)sCrm);
@@ -1779,7 +1824,7 @@ template <typename Real>
 void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t s, const SideStream& side)
 {
     const int ncell = a.M.ncell;
-    cudaMemsetAsync(a.cellWork, 0, 8 * sizeof(int), s);
+    cudaMemsetAsync(a.cellWork, 0, kWorkWords * sizeof(int), s);
     int gc = (ncell + 255) / 256;
     if (gc > L.smCount * 8) gc = L.smCount * 8;
     classify_kernel<Real><<<gc > 0 ? gc : 1, 256, 0, s>>>(a);

@@ -72,9 +72,9 @@ struct StepArgs {
     int* cellPairs;           // [ncell] candidate pair count of the step (classify pass)
     double* cellCons;         // [ncell] majorant term of the pair count (classify pass)
     int* cellList;            // [2*ncell] small, big and giant cells of the collision pass
-    int4* cellItem;           // [ncell] large cells of the collision pass: cell, start, count, pairs
-    double2* cellItemC;       // [ncell] the same items' majorant term and crmax
-    int* cellWork;            // [8] list lengths and hand-out counters of the cell pass
+    int4* cellItem;           // [2*ncell] large cells of the collision pass: cell, start, count, pairs
+    double2* cellItemC;       // [2*ncell] the same items' majorant term and crmax
+    int* cellWork;            // [16] list lengths and hand-out counters of the cell pass
     int* errorWord;
 };
 
