@@ -5,6 +5,7 @@
 #include "dsmc_gpu.h"
 #include "dsmc_meshio.h"
 #include "dsmc_kernels.cuh"
+#include "dsmc_hostlink.h"
 #include "dsmc_hostpack.h"
 
 #include <algorithm>
@@ -176,11 +177,8 @@ struct Engine {
     cudaEvent_t ev[6] = {};
     double stageMs[5] = {0, 0, 0, 0, 0};
     int64_t timedSteps = 0;
-    // pinned host chunks that pageable upload arrays pass through (allocated
-    // on the first such upload), and the events of their last copies
-    static constexpr size_t kHostStage = size_t(64) << 20;
-    void* hostStage[2] = {nullptr, nullptr};
-    cudaEvent_t stageEv[2] = {nullptr, nullptr};
+    HostLink link;                 // pageable host arrays to and from the device
+    char* traceWork = nullptr;     // dsmc_trace's device memory, for kTraceChunk particles at a time
 
     ~Engine() { release(); }
 
@@ -191,10 +189,7 @@ struct Engine {
             if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         for (auto& e : ev)
             if (e) { cudaEventDestroy(e); e = nullptr; }
-        for (int b = 0; b < 2; ++b) {
-            if (stageEv[b]) { cudaEventDestroy(stageEv[b]); stageEv[b] = nullptr; }
-            if (hostStage[b]) { cudaFreeHost(hostStage[b]); hostStage[b] = nullptr; }
-        }
+        link.release();
         for (void* p : allocs) cudaFree(p);
         allocs.clear();
         if (side.forked) { cudaEventDestroy(side.forked); side.forked = nullptr; }
@@ -1338,36 +1333,6 @@ struct Engine {
         return a.type == cudaMemoryTypeHost;
     }
 
-    // Host -> device on the handle's stream: pinned memory in one copy;
-    // pageable memory through the two pinned chunks, the host copy of the
-    // next chunk overlapping the transfer of the last. The source may be
-    // reused once the stream has been synchronised.
-    bool h2d(void* dst, const void* src, size_t bytes)
-    {
-        if (bytes == 0) return true;
-        if (hostPinned(src)) return cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), "upload");
-        for (int b = 0; b < 2; ++b) {
-            if (!hostStage[b] && !cuda(cudaHostAlloc(&hostStage[b], kHostStage, cudaHostAllocDefault), "pinned staging"))
-                return false;
-            if (!stageEv[b] && !cuda(cudaEventCreateWithFlags(&stageEv[b], cudaEventDisableTiming), "staging event"))
-                return false;
-        }
-        const char* s = static_cast<const char*>(src);
-        char* d = static_cast<char*>(dst);
-        const int nthreads = hostpack::threads_for((int64_t)(kHostStage / 8));
-        size_t j = 0;
-        for (size_t off = 0; off < bytes; off += kHostStage, ++j) {
-            const int b = (int)(j & 1);
-            const size_t len = std::min(kHostStage, bytes - off);
-            if (!cuda(cudaEventSynchronize(stageEv[b]), "staging wait")) return false;
-            hostpack::parallel_copy(hostStage[b], s + off, len, nthreads);
-            if (!cuda(cudaMemcpyAsync(d + off, hostStage[b], len, cudaMemcpyHostToDevice, stream), "upload") ||
-                !cuda(cudaEventRecord(stageEv[b], stream), "staging event"))
-                return false;
-        }
-        return true;
-    }
-
     // Upload of particles already in cell-major order (the order of the
     // reference's per-cell buckets, and of dsmc_download_particles): the cell
     // ids go up first and a kernel checks them and lays out start[]; the
@@ -1378,7 +1343,18 @@ struct Engine {
     int uploadCellMajor(int64_t n, const double* const src[7], const int32_t* cell)
     {
         int* dCell = static_cast<int*>(buf[cur][7]);
-        if (!h2d(dCell, cell, (size_t)n * sizeof(int))) return -1;
+        if (!cuda(link.ensure(device, stream), "pinned staging")) return -1;
+        if (hostPinned(cell)) {
+            if (!cuda(cudaMemcpyAsync(dCell, cell, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, stream), "upload")) return -1;
+        } else if (!cuda(link.in(1, &n,
+                                 [&](const HostLink::Block& b) { std::memcpy(b.host, cell + b.off, (size_t)b.len * 4); },
+                                 [&](const HostLink::Block& b) {
+                                     return cudaMemcpyAsync(dCell + b.off, b.host, (size_t)b.len * 4,
+                                                            cudaMemcpyHostToDevice, stream);
+                                 }),
+                         "upload")) {
+            return -1;
+        }
         if (!cuda(cudaMemsetAsync(uploadFlag, 0, sizeof(int), stream), "upload flag")) return -1;
         launch_upload_check(dCell, (int)n, ncell, uploadFlag, start[cur], stream);
         int flags = 0;
@@ -1391,26 +1367,49 @@ struct Engine {
             return -1;
         }
         if (flags & 2) return 0;
-        if (precision != DSMC_PRECISION_MIXED) {
-            for (int k = 0; k < 7; ++k)
-                if (!h2d(buf[cur][k], src[k], (size_t)n * sizeof(double))) return -1;
-            return 1;
-        }
-        // device chunks of the FP64 columns: the x and y arrays of the other
-        // buffer (capacity FP32 slots each, capacity / 2 FP64 values)
+        const bool mixed = precision == DSMC_PRECISION_MIXED;
+        // pinned columns in place: as they are, or through device chunks of
+        // FP64 values, the x and y arrays of the other buffer (capacity FP32
+        // slots each, capacity / 2 FP64 values)
+        int col[7], ncol = 0;
+        int64_t len[7];
         const int64_t m = std::max<int64_t>(1, capacity / 2);
         double* dstage[2] = {static_cast<double*>(buf[cur ^ 1][0]), static_cast<double*>(buf[cur ^ 1][1])};
         int64_t j = 0;
         for (int k = 0; k < 7; ++k) {
-            float* out = static_cast<float*>(buf[cur][k]);
-            for (int64_t off = 0; off < n; off += m, ++j) {
-                const int64_t len = std::min(m, n - off);
-                double* ds = dstage[j & 1];
-                if (!h2d(ds, src[k] + off, (size_t)len * sizeof(double))) return -1;
-                launch_upload_convert(ds, dCell + off, M.cellCenter, k, out + off, (int)len, stream);
+            if (!hostPinned(src[k])) {
+                col[ncol] = k;
+                len[ncol++] = n;
+            } else if (!mixed) {
+                if (!cuda(cudaMemcpyAsync(buf[cur][k], src[k], (size_t)n * sizeof(double), cudaMemcpyHostToDevice, stream), "upload"))
+                    return -1;
+            } else {
+                float* out = static_cast<float*>(buf[cur][k]);
+                for (int64_t off = 0; off < n; off += m, ++j) {
+                    const int64_t c = std::min(m, n - off);
+                    double* ds = dstage[j & 1];
+                    if (!cuda(cudaMemcpyAsync(ds, src[k] + off, (size_t)c * sizeof(double), cudaMemcpyHostToDevice, stream), "upload"))
+                        return -1;
+                    launch_upload_convert(ds, dCell + off, M.cellCenter, k, out + off, (int)c, stream);
+                }
             }
         }
-        return cuda(cudaGetLastError(), "upload convert") ? 1 : -1;
+        // the pageable ones
+        const cudaError_t e = link.in(
+            ncol, len,
+            [&](const HostLink::Block& b) { std::memcpy(b.host, src[col[b.col]] + b.off, (size_t)b.len * 8); },
+            [&](const HostLink::Block& b) {
+                const int k = col[b.col];
+                if (!mixed)
+                    return cudaMemcpyAsync(static_cast<double*>(buf[cur][k]) + b.off, b.host, (size_t)b.len * 8,
+                                           cudaMemcpyHostToDevice, stream);
+                const cudaError_t c = cudaMemcpyAsync(b.dev, b.host, (size_t)b.len * 8, cudaMemcpyHostToDevice, stream);
+                if (c != cudaSuccess) return c;
+                launch_upload_convert(reinterpret_cast<double*>(b.dev), dCell + b.off, M.cellCenter, k,
+                                      static_cast<float*>(buf[cur][k]) + b.off, (int)b.len, stream);
+                return cudaGetLastError();
+            });
+        return cuda(e, "upload") && cuda(cudaGetLastError(), "upload convert") ? 1 : -1;
     }
 
     bool uploadParticles(int64_t n, const double* px, const double* py, const double* pz, const double* vx,
@@ -1440,22 +1439,26 @@ struct Engine {
         haveParticles = false;
         if (!ensureCapacity(need)) return false;
         const bool mixed = precision == DSMC_PRECISION_MIXED;
-        std::vector<char> hb((size_t)n * 8);
-        for (int k = 0; k < 7; ++k) {
-            if (mixed)
-                hostpack::gather_convert<float>(n, order.data(), src[k], cell, k < 3 ? cellCenterHost.data() : nullptr, k,
-                                                reinterpret_cast<float*>(hb.data()), nthreads);
-            else
-                hostpack::gather_convert<double>(n, order.data(), src[k], cell, nullptr, k,
-                                                 reinterpret_cast<double*>(hb.data()), nthreads);
-            if (n > 0 && (!cuda(cudaMemcpyAsync(buf[cur][k], hb.data(), (size_t)n * realSize(), cudaMemcpyHostToDevice, stream), "upload particles") ||
-                          !cuda(cudaStreamSynchronize(stream), "sync")))
-                return false;
-        }
-        std::vector<int> hc((size_t)n);
-        hostpack::gather_cells(n, order.data(), cell, hc.data(), nthreads);
-        if (n > 0 && !cuda(cudaMemcpyAsync(buf[cur][7], hc.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, stream), "upload cells"))
-            return false;
+        if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
+        // the seven columns and the cell ids, gathered block by block
+        int64_t len[8];
+        std::fill(len, len + 8, n);
+        const size_t rs = realSize();
+        const cudaError_t ue = link.in(
+            8, len,
+            [&](const HostLink::Block& b) {
+                const int64_t* o = order.data() + b.off;
+                const double* shift = mixed && b.col < 3 ? cellCenterHost.data() : nullptr;
+                if (b.col == 7) hostpack::gather_cells(b.len, o, cell, reinterpret_cast<int*>(b.host), 1);
+                else if (mixed) hostpack::gather_convert<float>(b.len, o, src[b.col], cell, shift, b.col, reinterpret_cast<float*>(b.host), 1);
+                else hostpack::gather_convert<double>(b.len, o, src[b.col], cell, nullptr, b.col, reinterpret_cast<double*>(b.host), 1);
+            },
+            [&](const HostLink::Block& b) {
+                const size_t es = b.col == 7 ? sizeof(int) : rs;
+                return cudaMemcpyAsync(static_cast<char*>(buf[cur][b.col]) + (size_t)b.off * es, b.host, (size_t)b.len * es,
+                                       cudaMemcpyHostToDevice, stream);
+            });
+        if (!cuda(ue, "upload particles")) return false;
         if (!cuda(cudaMemcpyAsync(start[cur], st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice, stream), "upload start"))
             return false;
         return finishUpload(n);
@@ -1687,26 +1690,137 @@ struct Engine {
         int nl = 0;
         if (!nLiveHost(nl)) return false;
         if (n != nl) return fail("particle count mismatch: call dsmc_particle_count first");
-        std::vector<int> hc((size_t)n);
-        if (n > 0 && !cuda(cudaMemcpy(hc.data(), buf[cur][7], (size_t)n * sizeof(int), cudaMemcpyDeviceToHost), "cells"))
-            return false;
+        if (n == 0) return true;
         double* dst[7] = {px, py, pz, vx, vy, vz, ir};
         const bool mixed = precision == DSMC_PRECISION_MIXED;
-        std::vector<char> hb((size_t)n * 8);
-        const int nthreads = hostpack::threads_for(n);
-        for (int k = 0; k < 7; ++k) {
-            if (!dst[k] || n == 0) continue;
-            if (!cuda(cudaMemcpy(hb.data(), buf[cur][k], (size_t)n * realSize(), cudaMemcpyDeviceToHost), "particles"))
-                return false;
-            if (mixed)
-                hostpack::widen<float>(n, reinterpret_cast<const float*>(hb.data()), hc.data(),
-                                       k < 3 ? cellCenterHost.data() : nullptr, k, dst[k], nthreads);
-            else
-                hostpack::widen<double>(n, reinterpret_cast<const double*>(hb.data()), hc.data(), nullptr, k, dst[k],
-                                        nthreads);
+        if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
+        int col[8], ncol = 0;
+        int64_t len[8];
+        for (int k = 0; k < 8; ++k)
+            if (k < 7 ? dst[k] != nullptr : cellOut != nullptr) {
+                col[ncol] = k;
+                len[ncol++] = n;
+            }
+        const int* dCell = static_cast<const int*>(buf[cur][7]);
+        // the mixed path's values are widened on the device
+        const cudaError_t e = link.out(
+            ncol, len,
+            [&](const HostLink::Block& b) {
+                const int k = col[b.col];
+                if (k == 7) return cudaMemcpyAsync(b.host, dCell + b.off, (size_t)b.len * 4, cudaMemcpyDeviceToHost, stream);
+                const void* from = static_cast<const double*>(buf[cur][k]) + b.off;
+                if (mixed) {
+                    launch_download_widen(static_cast<const float*>(buf[cur][k]) + b.off, dCell + b.off, M.cellCenter, k,
+                                          reinterpret_cast<double*>(b.dev), (int)b.len, stream);
+                    const cudaError_t c = cudaGetLastError();
+                    if (c != cudaSuccess) return c;
+                    from = b.dev;
+                }
+                return cudaMemcpyAsync(b.host, from, (size_t)b.len * 8, cudaMemcpyDeviceToHost, stream);
+            },
+            [&](const HostLink::Block& b) {
+                const int k = col[b.col];
+                if (k == 7) std::memcpy(cellOut + b.off, b.host, (size_t)b.len * 4);
+                else std::memcpy(dst[k] + b.off, b.host, (size_t)b.len * 8);
+            });
+        if (!cuda(e, "particles")) return false;
+        if (pid)
+            hostpack::parallel_for(n, hostpack::threads_for(n), [&](int64_t b, int64_t c, int) {
+                for (int64_t j = b; j < c; ++j) pid[j] = (uint32_t)j;
+            });
+        return true;
+    }
+
+    // The tracing check in chunks of kTraceChunk particles, so that its device
+    // memory (19 MB, kept on the handle from the first call) does not grow
+    // with n; the conversions between FP64 and the working precision run on
+    // the device.
+    static constexpr int64_t kTraceChunk = 1 << 17;
+    bool trace(int64_t n, const double* const src[7], const int32_t* cell, int stopAtWall, int32_t* const iout[5],
+               double* const fout[7])
+    {
+        const bool mixed = precision == DSMC_PRECISION_MIXED;
+        const size_t N = (size_t)kTraceChunk;
+        // six FP64 columns and dt each way, the cells, six result columns
+        if (!traceWork && !alloc(traceWork, N * (14 * 8 + 7 * 4), false)) return false;
+        if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
+        double* dIn = reinterpret_cast<double*>(traceWork);
+        double* dOut = dIn + 7 * N;
+        int* dCell = reinterpret_cast<int*>(dOut + 7 * N);
+        int* dI = dCell + N;
+        for (int64_t base = 0; base < n; base += kTraceChunk) {
+            const int64_t m = std::min(kTraceChunk, n - base);
+            int64_t len[12];
+            std::fill(len, len + 12, m);
+            // the cells first: the conversions of the others read them
+            cudaError_t ce = link.in(
+                1, len, [&](const HostLink::Block& b) { std::memcpy(b.host, cell + base + b.off, (size_t)b.len * 4); },
+                [&](const HostLink::Block& b) {
+                    return cudaMemcpyAsync(dCell + b.off, b.host, (size_t)b.len * 4, cudaMemcpyHostToDevice, stream);
+                });
+            if (ce == cudaSuccess)
+                ce = link.in(
+                    7, len,
+                    [&](const HostLink::Block& b) { std::memcpy(b.host, src[b.col] + base + b.off, (size_t)b.len * 8); },
+                    [&](const HostLink::Block& b) {
+                        // FP32 columns in the first half of their FP64 ones
+                        const bool narrow = mixed && b.col < 6;
+                        double* to = dIn + (size_t)b.col * N;
+                        const cudaError_t c = cudaMemcpyAsync(narrow ? b.dev : reinterpret_cast<char*>(to + b.off), b.host,
+                                                              (size_t)b.len * 8, cudaMemcpyHostToDevice, stream);
+                        if (c != cudaSuccess || !narrow) return c;
+                        launch_upload_convert(reinterpret_cast<double*>(b.dev), dCell + b.off, M.cellCenter, b.col,
+                                              reinterpret_cast<float*>(to) + b.off, (int)b.len, stream);
+                        return cudaGetLastError();
+                    });
+            if (!cuda(ce, "trace upload")) return false;
+            int* oi[6];
+            for (int k = 0; k < 6; ++k) oi[k] = dI + (size_t)k * N;
+            auto launch = [&](auto zero) {
+                using Real = decltype(zero);
+                const Real* in[6];
+                Real* out[6];
+                for (int k = 0; k < 6; ++k) {
+                    in[k] = reinterpret_cast<const Real*>(dIn + (size_t)k * N);
+                    out[k] = reinterpret_cast<Real*>(dOut + (size_t)k * N);
+                }
+                launch_trace_check<Real>(M, C, (int)base, (int)m, in[0], in[1], in[2], in[3], in[4], in[5], dIn + 6 * N,
+                                         dCell, stopAtWall, oi[0], oi[1], oi[2], oi[3], oi[4], oi[5], out[0], out[1],
+                                         out[2], out[3], out[4], out[5], dOut + 6 * N, counters, stream);
+            };
+            if (mixed) launch(0.0f);
+            else launch(0.0);
+            if (!cuda(cudaGetLastError(), "trace launch")) return false;
+            int col[12], ncol = 0;
+            for (int k = 0; k < 5; ++k)
+                if (iout[k]) col[ncol++] = k;
+            for (int k = 0; k < 7; ++k)
+                if (fout[k]) col[ncol++] = 5 + k;
+            ce = link.out(
+                ncol, len,
+                [&](const HostLink::Block& b) {
+                    const int k = col[b.col];
+                    if (k < 5)
+                        return cudaMemcpyAsync(b.host, oi[k] + b.off, (size_t)b.len * 4, cudaMemcpyDeviceToHost, stream);
+                    const double* col64 = dOut + (size_t)(k - 5) * N;
+                    const void* from = col64 + b.off;
+                    if (mixed && k < 11) {
+                        // positions are relative to the cell the particle was last in
+                        launch_download_widen(reinterpret_cast<const float*>(col64) + b.off, oi[5] + b.off, M.cellCenter,
+                                              k - 5, reinterpret_cast<double*>(b.dev), (int)b.len, stream);
+                        const cudaError_t c = cudaGetLastError();
+                        if (c != cudaSuccess) return c;
+                        from = b.dev;
+                    }
+                    return cudaMemcpyAsync(b.host, from, (size_t)b.len * 8, cudaMemcpyDeviceToHost, stream);
+                },
+                [&](const HostLink::Block& b) {
+                    const int k = col[b.col];
+                    if (k < 5) std::memcpy(iout[k] + base + b.off, b.host, (size_t)b.len * 4);
+                    else std::memcpy(fout[k - 5] + base + b.off, b.host, (size_t)b.len * 8);
+                });
+            if (!cuda(ce, "trace out") || !cuda(cudaStreamSynchronize(stream), "trace sync")) return false;
         }
-        if (cellOut) std::memcpy(cellOut, hc.data(), (size_t)n * sizeof(int));
-        if (pid) for (int64_t j = 0; j < n; ++j) pid[j] = (uint32_t)j;
         return true;
     }
 
@@ -2023,92 +2137,10 @@ try {
     if (!px || !py || !pz || !vx || !vy || !vz || !dt || !cell) return DSMC_E_INVALID;
     for (int64_t i = 0; i < n; ++i)
         if (cell[i] < 0 || cell[i] >= e.ncell) { e.err = "trace: cell id out of range"; return DSMC_E_INVALID; }
-    const bool mixed = e.precision == DSMC_PRECISION_MIXED;
-    const size_t rs = mixed ? 4 : 8;
-    // device scratch of this call: every failed allocation is recorded, and
-    // whatever was allocated is freed on every way out
-    struct DeviceTemps {
-        std::vector<void*> ptrs;
-        bool failed = false;
-        void* alloc(size_t bytes)
-        {
-            ptrs.reserve(ptrs.size() + 1);
-            void* q = nullptr;
-            if (cudaMalloc(&q, std::max<size_t>(bytes, 1)) != cudaSuccess) {
-                failed = true;
-                (void)cudaGetLastError();
-                return nullptr;
-            }
-            ptrs.push_back(q);
-            return q;
-        }
-        ~DeviceTemps()
-        {
-            for (void* q : ptrs) cudaFree(q);
-        }
-    } tmp;
-    auto dal = [&](size_t bytes) -> void* { return tmp.alloc(bytes); };
-    void* dIn[6];
-    void* dOut[6];
-    for (int k = 0; k < 6; ++k) {
-        dIn[k] = dal((size_t)n * rs);
-        dOut[k] = dal((size_t)n * rs);
-    }
-    double* dDt = (double*)dal((size_t)n * 8);
-    double* dODt = (double*)dal((size_t)n * 8);
-    int* dCell = (int*)dal((size_t)n * 4);
-    int* dI[6];
-    for (int k = 0; k < 6; ++k) dI[k] = (int*)dal((size_t)n * 4);
-    if (tmp.failed) { e.err = "trace: device allocation failed"; return DSMC_E_NOMEM; }
-    const double* src[6] = {px, py, pz, vx, vy, vz};
-    std::vector<char> hb((size_t)n * 8);
-    bool ok = true;
-    for (int k = 0; k < 6 && ok; ++k) {
-        for (int64_t i = 0; i < n; ++i) {
-            double v = src[k][i];
-            if (mixed) {
-                if (k < 3) v -= e.cellCenterHost[(size_t)cell[i] * 3 + k];
-                reinterpret_cast<float*>(hb.data())[i] = (float)v;
-            } else {
-                reinterpret_cast<double*>(hb.data())[i] = v;
-            }
-        }
-        ok = e.cuda(cudaMemcpy(dIn[k], hb.data(), (size_t)n * rs, cudaMemcpyHostToDevice), "trace upload");
-    }
-    ok = ok && e.cuda(cudaMemcpy(dDt, dt, (size_t)n * 8, cudaMemcpyHostToDevice), "trace dt");
-    ok = ok && e.cuda(cudaMemcpy(dCell, cell, (size_t)n * 4, cudaMemcpyHostToDevice), "trace cells");
-    if (ok) {
-        if (mixed)
-            dsmc::launch_trace_check<float>(e.M, e.C, (int)n, (float*)dIn[0], (float*)dIn[1], (float*)dIn[2],
-                                            (float*)dIn[3], (float*)dIn[4], (float*)dIn[5], dDt, dCell, stop_at_wall,
-                                            dI[0], dI[1], dI[2], dI[3], dI[4], dI[5], (float*)dOut[0], (float*)dOut[1],
-                                            (float*)dOut[2], (float*)dOut[3], (float*)dOut[4], (float*)dOut[5], dODt,
-                                            e.counters, e.stream);
-        else
-            dsmc::launch_trace_check<double>(e.M, e.C, (int)n, (double*)dIn[0], (double*)dIn[1], (double*)dIn[2],
-                                             (double*)dIn[3], (double*)dIn[4], (double*)dIn[5], dDt, dCell,
-                                             stop_at_wall, dI[0], dI[1], dI[2], dI[3], dI[4], dI[5], (double*)dOut[0],
-                                             (double*)dOut[1], (double*)dOut[2], (double*)dOut[3], (double*)dOut[4],
-                                             (double*)dOut[5], dODt, e.counters, e.stream);
-        ok = e.cuda(cudaGetLastError(), "trace launch") && e.cuda(cudaStreamSynchronize(e.stream), "trace sync");
-    }
-    std::vector<int> last((size_t)n);
+    const double* src[7] = {px, py, pz, vx, vy, vz, dt};
     int32_t* iout[5] = {out_cell, out_ifout, out_face, out_tri, out_ncross};
-    for (int k = 0; k < 5 && ok; ++k)
-        if (iout[k]) ok = e.cuda(cudaMemcpy(iout[k], dI[k], (size_t)n * 4, cudaMemcpyDeviceToHost), "trace out");
-    ok = ok && e.cuda(cudaMemcpy(last.data(), dI[5], (size_t)n * 4, cudaMemcpyDeviceToHost), "trace last");
-    double* fout[6] = {out_px, out_py, out_pz, out_vx, out_vy, out_vz};
-    for (int k = 0; k < 6 && ok; ++k) {
-        if (!fout[k]) continue;
-        ok = e.cuda(cudaMemcpy(hb.data(), dOut[k], (size_t)n * rs, cudaMemcpyDeviceToHost), "trace out");
-        for (int64_t i = 0; i < n && ok; ++i) {
-            double v = mixed ? (double)reinterpret_cast<float*>(hb.data())[i] : reinterpret_cast<double*>(hb.data())[i];
-            if (mixed && k < 3) v = e.cellCenterHost[(size_t)last[(size_t)i] * 3 + k] + v;
-            fout[k][i] = v;
-        }
-    }
-    if (ok && out_dt) ok = e.cuda(cudaMemcpy(out_dt, dODt, (size_t)n * 8, cudaMemcpyDeviceToHost), "trace dt out");
-    return status_of(e, ok);
+    double* fout[7] = {out_px, out_py, out_pz, out_vx, out_vy, out_vz, out_dt};
+    return status_of(e, e.trace(n, src, cell, stop_at_wall, iout, fout));
 }
 DSMC_CATCH(h ? &h->e.err : nullptr)
 

@@ -2262,11 +2262,28 @@ void launch_upload_convert(const double* in, const int* cell, const double* cent
     upload_convert_kernel<<<g, 256, 0, s>>>(in, cell, center, comp, out, n);
 }
 
+__global__ void download_widen_kernel(const float* __restrict__ in, const int* __restrict__ cell,
+                                      const double* __restrict__ center, int comp, double* __restrict__ out, int n)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        double v = (double)in[i];
+        if (comp < 3) v = da(center[(size_t)cell[i] * 3 + comp], v);
+        out[i] = v;
+    }
+}
+
+void launch_download_widen(const float* in, const int* cell, const double* center, int comp, double* out, int n,
+                           cudaStream_t s)
+{
+    const int g = max(1, min((n + 255) / 256, 148 * 16));
+    download_widen_kernel<<<g, 256, 0, s>>>(in, cell, center, comp, out, n);
+}
+
 // ===========================================================================
 // tracing check (dsmc_trace)
 // ===========================================================================
 template <typename Real>
-__global__ void trace_check_kernel(DevMesh M, DevConsts C, int n, const Real* px, const Real* py, const Real* pz,
+__global__ void trace_check_kernel(DevMesh M, DevConsts C, int first, int n, const Real* px, const Real* py, const Real* pz,
                                    const Real* vx, const Real* vy, const Real* vz, const double* dt,
                                    const int* cell, int stopAtWall, int* oCell, int* oIfout, int* oFace,
                                    int* oTri, int* oNcross, int* oLast, Real* ox, Real* oy, Real* oz, Real* ovx,
@@ -2285,7 +2302,7 @@ __global__ void trace_check_kernel(DevMesh M, DevConsts C, int n, const Real* px
         p.v[0] = vx[i]; p.v[1] = vy[i]; p.v[2] = vz[i];
         p.ir = (Real)0;
         Stream rs;
-        rs.init((uint32_t)i, 0u, kPurposeWall, C.seedLo, C.seedHi);
+        rs.init((uint32_t)(first + i), 0u, kPurposeWall, C.seedLo, C.seedHi);
         double dtleft = dt[i];
         TraceLog log{-1, 0, 0};
         const int out = trace_particle<Real>(M, C, p, c, -1, -1, dtleft, rs, 0, nullptr, cnt, stopAtWall != 0, &log);
@@ -2309,7 +2326,7 @@ __global__ void trace_check_kernel(DevMesh M, DevConsts C, int n, const Real* px
 }
 
 template <typename Real>
-void launch_trace_check(const DevMesh& M, const DevConsts& C, int n, const Real* px, const Real* py, const Real* pz,
+void launch_trace_check(const DevMesh& M, const DevConsts& C, int first, int n, const Real* px, const Real* py, const Real* pz,
                         const Real* vx, const Real* vy, const Real* vz, const double* dt, const int* cell,
                         int stopAtWall, int* oCell, int* oIfout, int* oFace, int* oTri, int* oNcross, int* oLast,
                         Real* ox, Real* oy, Real* oz, Real* ovx, Real* ovy, Real* ovz, double* odt,
@@ -2317,7 +2334,7 @@ void launch_trace_check(const DevMesh& M, const DevConsts& C, int n, const Real*
 {
     int g = (n + 255) / 256;
     if (g > 4096) g = 4096;
-    trace_check_kernel<Real><<<g > 0 ? g : 1, 256, 0, s>>>(M, C, n, px, py, pz, vx, vy, vz, dt, cell, stopAtWall,
+    trace_check_kernel<Real><<<g > 0 ? g : 1, 256, 0, s>>>(M, C, first, n, px, py, pz, vx, vy, vz, dt, cell, stopAtWall,
                                                            oCell, oIfout, oFace, oTri, oNcross, oLast, ox, oy, oz,
                                                            ovx, ovy, ovz, odt, counters);
 }
@@ -2331,7 +2348,7 @@ void launch_trace_check(const DevMesh& M, const DevConsts& C, int n, const Real*
     template void launch_fill<Real>(const StepArgs<Real>&, const FillParams&, const int*, const LaunchShape&,    \
                                     cudaStream_t);                                                               \
     template cudaError_t prepare_kernels<Real>();                                                                \
-    template void launch_trace_check<Real>(const DevMesh&, const DevConsts&, int, const Real*, const Real*,       \
+    template void launch_trace_check<Real>(const DevMesh&, const DevConsts&, int, int, const Real*, const Real*,  \
                                            const Real*, const Real*, const Real*, const Real*, const double*,    \
                                            const int*, int, int*, int*, int*, int*, int*, int*, Real*, Real*,    \
                                            Real*, Real*, Real*, Real*, double*, unsigned long long*, cudaStream_t);

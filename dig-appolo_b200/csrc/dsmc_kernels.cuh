@@ -158,11 +158,15 @@ void launch_upload_convert(const double* in, const int* cell, const double* cent
 // where the mesh has no such blocks, and their packing.
 size_t geo_floats(const DevMesh& M);
 void launch_pack_geo(const DevMesh& M, float4* geo, cudaStream_t s);
+// out[i] = (center[cell[i] * 3 + comp] for comp < 3) + (double)in[i]
+void launch_download_widen(const float* in, const int* cell, const double* center, int comp, double* out, int n,
+                           cudaStream_t s);
 template <typename Real> cudaError_t prepare_kernels();
 void launch_macro(const DevMesh& M, const DevConsts& C, const double* acc, int set, double count,
                   double* out, int ncell, cudaStream_t s);
+// first: the number of the first particle (its random stream)
 template <typename Real>
-void launch_trace_check(const DevMesh& M, const DevConsts& C, int n, const Real* px, const Real* py,
+void launch_trace_check(const DevMesh& M, const DevConsts& C, int first, int n, const Real* px, const Real* py,
                         const Real* pz, const Real* vx, const Real* vy, const Real* vz,
                         const double* dt, const int* cell, int stopAtWall, int* oCell, int* oIfout,
                         int* oFace, int* oTri, int* oNcross, int* oLast, Real* ox, Real* oy, Real* oz,

@@ -170,14 +170,14 @@ extern "C" int dsmc_trace_noalloc(DsmcHandle* h, int64_t n, const double* px, co
         if (mixed) {
             const float* wi = static_cast<const float*>(dWorkIn);
             float* wo = static_cast<float*>(dWorkOut);
-            dsmc::launch_trace_check<float>(M, Cst, ni, wi, wi + N, wi + 2 * N, wi + 3 * N, wi + 4 * N, wi + 5 * N,
+            dsmc::launch_trace_check<float>(M, Cst, 0, ni, wi, wi + N, wi + 2 * N, wi + 3 * N, wi + 4 * N, wi + 5 * N,
                                             dIn + 6 * N, dCell, stop_at_wall, oi[0], oi[1], oi[2], oi[3], oi[4], oi[5],
                                             wo, wo + N, wo + 2 * N, wo + 3 * N, wo + 4 * N, wo + 5 * N, dOut + 6 * N,
                                             dsmc::engine_counters(h), s);
         } else {
             const double* wi = static_cast<const double*>(dWorkIn);
             double* wo = static_cast<double*>(dWorkOut);
-            dsmc::launch_trace_check<double>(M, Cst, ni, wi, wi + N, wi + 2 * N, wi + 3 * N, wi + 4 * N, wi + 5 * N,
+            dsmc::launch_trace_check<double>(M, Cst, 0, ni, wi, wi + N, wi + 2 * N, wi + 3 * N, wi + 4 * N, wi + 5 * N,
                                              dIn + 6 * N, dCell, stop_at_wall, oi[0], oi[1], oi[2], oi[3], oi[4], oi[5],
                                              wo, wo + N, wo + 2 * N, wo + 3 * N, wo + 4 * N, wo + 5 * N, dOut + 6 * N,
                                              dsmc::engine_counters(h), s);

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 
@@ -172,6 +173,28 @@ def _ptr(a):
     return None if a is None else a.ctypes.data_as(C.c_void_p)
 
 
+_rows_pool = None
+
+
+def _rows(cols):
+    """np.stack(cols, 1), by several threads for long columns (the strided
+    copy and the page faults of the new array are most of a download)."""
+    global _rows_pool
+    n = cols[0].shape[0]
+    if n < 1 << 16:
+        return np.stack(cols, 1)
+    if _rows_pool is None:
+        _rows_pool = ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1)))
+    out = np.empty((n, len(cols)), dtype=cols[0].dtype)
+
+    def part(a):
+        for k, c in enumerate(cols):
+            out[a:a + (1 << 16), k] = c[a:a + (1 << 16)]
+
+    list(_rows_pool.map(part, range(0, n, 1 << 16)))
+    return out
+
+
 class DsmcError(RuntimeError):
     pass
 
@@ -257,7 +280,7 @@ class Case:
         pid = np.empty(n, dtype=np.uint32)
         self._check(self.lib.dsmc_download_particles(self.h, n, *[_ptr(a) for a in arrs], _ptr(cell), _ptr(pid)),
                     "dsmc_download_particles")
-        return (np.stack(arrs[:3], 1), np.stack(arrs[3:6], 1), arrs[6], cell)
+        return (_rows(arrs[:3]), _rows(arrs[3:6]), arrs[6], cell)
 
     # -- stages -----------------------------------------------------------------
     def step(self, istep: int, stages: int = STAGE_ALL):
@@ -362,7 +385,7 @@ class Case:
                        *[_ptr(a) for a in oi], *[_ptr(a) for a in of]),
                     "dsmc_trace_noalloc" if noalloc else "dsmc_trace")
         return {"cell": oi[0], "ifout": oi[1], "face": oi[2], "tri": oi[3], "ncross": oi[4],
-                "x": np.stack(of[:3], 1), "v": np.stack(of[3:6], 1), "dt": of[6]}
+                "x": _rows(of[:3]), "v": _rows(of[3:6]), "dt": of[6]}
 
     def fill_initial(self, ppc_mean: float, seed: int = 0):
         """The reference's initial fill on the device (dsmc_fill_initial)."""
