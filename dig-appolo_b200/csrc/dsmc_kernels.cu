@@ -1243,101 +1243,71 @@ __device__ __forceinline__ Real warp_max(Real m)
     return m;
 }
 
-// NTC collisions of one cell by one warp, in place in the particle buffer,
-// for cells beyond every shared-memory arena. The pairs run as a sliding
-// window: every lane holds one pending pair and claims both its particles
-// with the pair index (atomicMin); a pair whose index is the lowest claim on
-// both particles goes, and its lane takes the next unassigned pair. Pairs are
-// handed out in increasing order, so a pair goes only after every lower pair
-// that shares a particle with it, and the result equals running the pairs one
-// after another. The lowest pending pair always goes, so the loop ends after
-// at most npairs rounds. The claims sit in the cell-id slots of the cell and
-// are replaced by the cell id at the end.
-template <typename Real>
-__device__ void collide_cell_in_place(const PBuf<Real>& buf, int s0, int n, int c, int npairs, double consCrm,
-                                      double crm0, const StepArgs<Real>& a, int istep, uint32_t& collOut)
-{
-    const int lane = threadIdx.x & 31;
-    int* claim = buf.cell + s0;
-    Real* const v[4] = {buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0};
-    for (int k = lane; k < n; k += 32) claim[k] = INT_MAX;
-    __syncwarp();
-    Real crmLocal = (Real)0;
-    const Real crm0r = (Real)crm0;
-    const unsigned below = (1u << lane) - 1u;
-    int next = 0;     // first pair not yet handed out (same in every lane)
-    int j = -1;       // this lane's pending pair
-    int k1 = 0, k2 = 0;
-    PairDraw d;
-    for (;;) {
-        const unsigned idle = __ballot_sync(kFull, j < 0);
-        if (j < 0) {
-            const int jj = next + __popc(idle & below);
-            if (jj < npairs) {
-                j = jj;
-                d = pair_draw(c, istep, j, n, a.C, k1, k2);
-            }
-        }
-        next = min(npairs, next + __popc(idle));
-        if (__ballot_sync(kFull, j >= 0) == 0u) break;
-        if (j >= 0) {
-            atomicMin(&claim[k1], j);
-            atomicMin(&claim[k2], j);
-        }
-        __syncwarp();
-        const bool go = j >= 0 && claim[k1] == j && claim[k2] == j;
-        __syncwarp();
-        if (go) {
-            PState<Real> p{v[0][k1], v[1][k1], v[2][k1], v[3][k1]}, q{v[0][k2], v[1][k2], v[2][k2], v[3][k2]};
-            if (pair_collide<Real>(p, q, c, istep, j, d.b0.z, d.b0.w, a.C, consCrm, crm0r, true, crmLocal)) {
-                v[0][k1] = p.x; v[1][k1] = p.y; v[2][k1] = p.z; v[3][k1] = p.i;
-                v[0][k2] = q.x; v[1][k2] = q.y; v[2][k2] = q.z; v[3][k2] = q.i;
-                ++collOut;
-            }
-            claim[k1] = INT_MAX;
-            claim[k2] = INT_MAX;
-            j = -1;
-        }
-        __syncwarp();
-    }
-    const double m = largest_speed(warp_max(crmLocal));
-    if (lane == 0 && m > crm0) a.crmax[c] = m;
-    for (int k = lane; k < n; k += 32) claim[k] = c;
-    __syncwarp();
-}
-
 // The collision pass over the sorted buffer (collisionDSMC,
 // src/ProcessDSMC.cpp:2621-2665). Cells are classed first (classify_kernel):
-// - small cells (at most kSmallMax particles and kSmallPairs pairs): 32 at a
-//   time per warp, lane l owning one cell and running its pairs alone, with the particles'
-//   velocities and internal energies in shared memory at slot k * 32 + l
-//   (lane l's slots sit in bank l, so the lanes never conflict);
+// - small cells (at most CellShape::small particles and kSmallPairs pairs): 32
+//   at a time per warp, lane l owning one cell and running its pairs alone, with
+//   the particles' velocities and internal energies in shared memory at slot
+//   k * 32 + l (lane l's slots sit in bank l, so the lanes never conflict); when
+//   all cells together are few enough for half a warp each, as large cells;
 // - large cells: two at a time per warp, staged in shared memory
 //   (collide_kernel), those of the most rounds first;
+// - middle cells (more than kMiddlePairs pairs): as big cells when every one
+//   of them finds a free block, as large cells otherwise;
 // - big cells (more particles than a warp's arena, or more pairs than
 //   kBigPairs) and giants (more pairs than kGiantPairs, handed out first):
-//   one at a time by a block of 512 threads (collide_big_kernel), beside the
+//   one at a time by a block of 256 threads (collide_big_kernel), beside the
 //   other kernel on the side stream.
 // A cell's result depends on nothing but the cell, so neither the warp or
 // block that takes it nor the order matters.
 //
 // What bounds it: a cell's pairs depend on each other through its particles,
-// so a cell is a chain of rounds, and the pass is as long as the longest
-// chain. With every cell run by one warp, 32 pairs a round at most, the few
-// compressed cells of a capsule (2,000 particles, 30,000-60,000 pairs) were
-// the whole pass. A block runs up to 512 pairs a round (n / 4 (1 - e^(-2048 / n))
-// of them go), in a tenth of the rounds. Next longest were cells of up to 16
-// particles with up to 900 pairs, one lane running one after another.
+// so a cell is a chain of rounds. Where cells are few, the pass is as long as
+// its longest chain; where they are many, it is bound by instruction issue
+// (of 32 lanes some 12 work) and by the warps that fit an SM.
+// - With every cell run by one warp, 32 pairs a round at most, the few
+//   compressed cells of a capsule (2,000 particles, 30,000-60,000 pairs) were
+//   the whole pass. A block runs up to 256 pairs a round, in a fifth of the
+//   rounds. Two blocks of 256 threads an SM, not one of 512: one's barriers are
+//   covered by the other (FP64 capsule of 63,500 cells, the step: 2,990 us
+//   with 512 threads, 2,750 with 2 x 256).
+// - A warp outdoes a block in throughput, so in a full device the blocks only
+//   get chains that would outlast the pass: with kBigPairs at 512 that
+//   capsule's step took 4,380 us, at 2,048 2,840. Where the blocks are free,
+//   they shorten the pass (6,080 cells: 52 -> 32 us).
+// - Cells of up to 16 particles can have 900 pairs, one lane running one after
+//   another. In a full device lanes still do best for those of up to 32 pairs
+//   (372,500 cells, the step: 4,280 us; with warps for those of more than 4
+//   particles 4,420); in an empty one they are the longest chain (760 cells:
+//   19.5 us, 9.1 by half warps).
+// - FP64 needs 36 bytes a particle: arenas of 376 let eight blocks (16 warps)
+//   into an SM, of 512 six (48,640 cells: 113 us with six, 91 with eight).
+// Arenas (FP32 20 KB, FP64 26 KB per block, plus the 1 KB the runtime reserves)
+// fill an SM's 228 KB.
 constexpr int kCellWarps = 2;                 // warps per block of collide_kernel
 constexpr int kSmallMax = 16;
-constexpr int kArena = 512;                   // staged particles per warp
-static_assert(32 * kSmallMax <= kArena, "small-cell slots must fit in the arena");
-constexpr int kBigThreads = 512;
-constexpr int kBigArena = 4096;               // staged particles per block of collide_big_kernel
-constexpr int kBigPairs = 1024;
+constexpr int kBigThreads = 256;
+constexpr int kBigPerSm = 2;                  // resident blocks of collide_big_kernel per SM
+constexpr int kBigArena = 2048;               // staged particles per block of collide_big_kernel
+constexpr int kBigPairs = 1024, kMiddlePairs = 512;
 constexpr int kBigLeast = 128;                // fewer particles give a block no more pairs a round than a warp
+template <typename Real>
+struct CellShape;
+template <>
+struct CellShape<float> {
+    static constexpr int arena = 512;         // staged particles per warp
+    static constexpr int blocks = 10;         // resident blocks of collide_kernel per SM
+    static constexpr int small = kSmallMax;   // particles of a small cell
+};
+template <>
+struct CellShape<double> {
+    static constexpr int arena = 376;
+    static constexpr int blocks = 8;
+    static constexpr int small = 12;
+};
 constexpr int kSmallPairs = 32;
 constexpr int kGiantPairs = 8192;
+constexpr int kStagedSum = 512;               // see pair_accept: FP32 cells beyond it add the squares in two roundings
 
 // shared memory of `slots` staged particles: their states and claims
 template <typename Real>
@@ -1345,6 +1315,9 @@ __host__ __device__ constexpr size_t arena_bytes(int slots)
 {
     return (size_t)slots * (4 * sizeof(Real) + sizeof(int));
 }
+static_assert(32 * CellShape<float>::small * 4 * sizeof(float) <= arena_bytes<float>(CellShape<float>::arena) &&
+                  32 * CellShape<double>::small * 4 * sizeof(double) <= arena_bytes<double>(CellShape<double>::arena),
+              "small-cell slots must fit in the arena");
 
 // particle states in shared memory, 16 bytes a load
 template <typename Real>
@@ -1381,6 +1354,18 @@ struct Arena<double> {
     {
         lo[k] = make_double2(p.x, p.y);
         hi[k] = make_double2(p.z, p.i);
+    }
+};
+
+// the states and claims of a cell run in place in the particle buffer
+template <typename Real>
+struct InPlace {
+    Real* v[4];
+    int* claim;
+    __device__ __forceinline__ PState<Real> get(int k) const { return {v[0][k], v[1][k], v[2][k], v[3][k]}; }
+    __device__ __forceinline__ void put(int k, const PState<Real>& p) const
+    {
+        v[0][k] = p.x; v[1][k] = p.y; v[2][k] = p.z; v[3][k] = p.i;
     }
 };
 
@@ -1421,17 +1406,31 @@ __device__ __forceinline__ void unstage_cell(const PBuf<Real>& buf, const Arena<
 
 // cellWork: [0..2] large counts by their rounds (more than kManyRounds, more
 //           than kSomeRounds, the rest), [3] small count, [4] big count, [5] giant
-//           count, [6] next large item, [7] next small, [8] next giant or big
+//           count, [6] next large item, [7] next small, [8] next giant or big,
+//           [9] middle count
 // cellList: small cells from the front of [0, ncell), big cells from its
 //           back, giants from the front of [ncell, 2 ncell)
 // cellItem: large cells, of many rounds from the front of [0, ncell), of some
-//           from its back, the rest from the front of [ncell, 2 ncell); handed
-//           out in this order, so that the longest chains start first
+//           from its back, the rest from the front of [ncell, 2 ncell), middle
+//           cells from its back; handed out middle, many, some, rest, so that
+//           the longest chains start first
 constexpr int kWorkWords = 16;
 constexpr int kManyRounds = 40, kSomeRounds = 12;
-__device__ __forceinline__ int large_slot(int it, int n0, int n1, int ncell)
+struct LargeLists {
+    int middle, many, some, all;   // counts; all: of the three and the rest
+    int small;                     // small cells that follow them, one item each
+    __device__ __forceinline__ int slot(int it, int ncell) const
+    {
+        if (it < middle) return 2 * ncell - 1 - it;
+        it -= middle;
+        return it < many ? it : it < many + some ? ncell - 1 - (it - many) : ncell + (it - many - some);
+    }
+};
+// Middle cells go to the blocks when every one of them finds a free block at
+// once, and to the warps otherwise.
+__device__ __forceinline__ bool middle_by_blocks(const int* work, int bigBlocks)
 {
-    return it < n0 ? it : it < n0 + n1 ? ncell - 1 - (it - n0) : ncell + (it - n0 - n1);
+    return work[4] + work[5] + work[9] <= bigBlocks;
 }
 template <typename Real>
 __global__ void classify_kernel(StepArgs<Real> a)
@@ -1460,23 +1459,24 @@ __global__ void classify_kernel(StepArgs<Real> a)
         if (n > 1 && np > 0 && consCrm > 0.0) {
             // a round runs about 13 pairs of a cell, n / 4 of one with few particles
             const int rounds = np / min(13, max(1, n >> 2));
-            if (n <= kSmallMax && np <= kSmallPairs) cls = 3;
+            if (n <= CellShape<Real>::small && np <= kSmallPairs) cls = 3;
             else if (np > kGiantPairs && n > kBigLeast) cls = 5;
-            else if (n > kArena || (np > kBigPairs && n > kBigLeast)) cls = 4;
+            else if (n > CellShape<Real>::arena || (np > kBigPairs && n > kBigLeast)) cls = 4;
+            else if (np > kMiddlePairs && n > kBigLeast) cls = 6;
             else cls = rounds > kManyRounds ? 0 : rounds > kSomeRounds ? 1 : 2;
         }
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
+        for (int k = 0; k < 7; ++k) {
             const unsigned m = __ballot_sync(kFull, cls == k);
             if (!m) continue;
             const int leader = __ffs(m) - 1;
             int b = 0;
-            if (lane == leader) b = atomicAdd(work + k, __popc(m));
+            if (lane == leader) b = atomicAdd(work + (k < 6 ? k : 9), __popc(m));
             b = __shfl_sync(kFull, b, leader);
             if (cls == k) {
                 const int pos = b + __popc(m & ((1u << lane) - 1u));
-                if (k < 3) {
-                    const int slot = k == 0 ? pos : k == 1 ? ncell - 1 - pos : ncell + pos;
+                if (k < 3 || k == 6) {
+                    const int slot = k == 0 ? pos : k == 1 ? ncell - 1 - pos : k == 2 ? ncell + pos : 2 * ncell - 1 - pos;
                     a.cellItem[slot] = make_int4(c, s0, n, np);
                     a.cellItemC[slot] = make_double2(consCrm, crm0);
                 } else {
@@ -1512,8 +1512,8 @@ __device__ __forceinline__ void copy_cell(const PBuf<Real>& buf, int s0, int n, 
 }
 
 // Collisions of staged large cells, two cells per warp at a time, both in
-// the warp's arena: channel 0's cell at slots [0, n0), channel 1's at
-// [kArena - n1, kArena); a cell that does not fit beside the other channel's
+// the warp's arena: channel 0's cell at its front, channel 1's at its
+// back; a cell that does not fit beside the other channel's
 // waits until that one is done. The pairs run as a sliding window: every
 // lane holds one pending pair of either cell and claims its two particles
 // with the pair index (atomicMin); a pair whose index is the lowest claim on
@@ -1530,10 +1530,11 @@ __device__ __forceinline__ void copy_cell(const PBuf<Real>& buf, int s0, int n, 
 // some 13 to 20 go a round, and of 16 about 13; each phase then runs once a
 // round for both cells.
 template <typename Real>
-__device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf, const Arena<Real>& A, int n0, int n1,
-                                  int nItems, int istep, uint32_t& colls)
+__device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf, const Arena<Real>& A,
+                                  const LargeLists& L, int istep, uint32_t& colls)
 {
-    constexpr int N = kArena;
+    constexpr int N = CellShape<Real>::arena;
+    const int nItems = L.all + L.small;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     int cc[2] = {-1, -1}, cbase[2] = {0, 0}, cs0[2] = {0, 0}, cn[2] = {0, 0}, cnp[2] = {0, 0}, cnext[2] = {0, 0};
@@ -1587,9 +1588,17 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
                     more = false;
                     break;
                 }
-                const int slot = large_slot(it, n0, n1, a.M.ncell);
-                const int4 rec = a.cellItem[slot];
-                const double2 rc = a.cellItemC[slot];
+                int4 rec;
+                double2 rc;
+                if (it < L.all) {
+                    const int slot = L.slot(it, a.M.ncell);
+                    rec = a.cellItem[slot];
+                    rc = a.cellItemC[slot];
+                } else {
+                    const int c = a.cellList[it - L.all], s0 = a.startA[c];
+                    rec = make_int4(c, s0, a.startA[c + 1] - s0, a.cellPairs[c]);
+                    rc = make_double2(a.cellCons[c], a.crmax[c]);
+                }
                 const int n = rec.z;
                 if (n > N) {   // never reached (classify lists no such cell): flag rather than overflow the arena
                     if (lane == 0) atomicOr(a.errorWord, kErrStageCell);
@@ -1644,24 +1653,31 @@ __device__ void collide_two_cells(const StepArgs<Real>& a, const PBuf<Real>& buf
     }
 }
 
-// Ten resident blocks (20 warps) per SM in FP32, six in FP64: the arenas
-// (20 and 36 KB per block plus the 1 KB the runtime reserves) fill the 228 KB.
 template <typename Real>
-__global__ void __launch_bounds__(kCellWarps * 32, sizeof(Real) == 4 ? 10 : 6) collide_kernel(StepArgs<Real> a)
+__global__ void __launch_bounds__(kCellWarps * 32, CellShape<Real>::blocks) collide_kernel(StepArgs<Real> a, int bigBlocks)
 {
     extern __shared__ __align__(16) unsigned char cellSmem[];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    unsigned char* const wsm = cellSmem + (size_t)wib * arena_bytes<Real>(kArena);
+    unsigned char* const wsm = cellSmem + (size_t)wib * arena_bytes<Real>(CellShape<Real>::arena);
     const int istep = a.ctl->istep;
     const PBuf<Real> buf = a.A;
     uint32_t colls = 0;
 
-    const int n0 = a.cellWork[0], n1 = a.cellWork[1], nLarge = n0 + n1 + a.cellWork[2], nSmall = a.cellWork[3];
-    if (nLarge > 0) collide_two_cells<Real>(a, buf, Arena<Real>(wsm, kArena), n0, n1, nLarge, istep, colls);
+    int nSmall = a.cellWork[3];
+    LargeLists L;
+    L.middle = middle_by_blocks(a.cellWork, bigBlocks) ? 0 : a.cellWork[9];
+    L.many = a.cellWork[0];
+    L.some = a.cellWork[1];
+    L.all = L.middle + L.many + L.some + a.cellWork[2];
+    // few enough cells for half a warp each: the small ones too, since one
+    // lane's pairs one after another take longer than a warp's rounds
+    L.small = L.all + nSmall <= (int)(gridDim.x * kCellWarps) * 2 ? nSmall : 0;
+    nSmall -= L.small;
+    if (L.all + L.small > 0) collide_two_cells<Real>(a, buf, Arena<Real>(wsm, CellShape<Real>::arena), L, istep, colls);
 
     // ---- small cells, 32 per warp, one lane each
-    constexpr int kSmallSlots = 32 * kSmallMax;
+    constexpr int kSmallSlots = 32 * CellShape<Real>::small;
     Real* const sv = reinterpret_cast<Real*>(wsm);
     Real* const stage[4] = {sv, sv + kSmallSlots, sv + 2 * kSmallSlots, sv + 3 * kSmallSlots};
     const int* start = a.startA;
@@ -1696,25 +1712,91 @@ __global__ void __launch_bounds__(kCellWarps * 32, sizeof(Real) == 4 ? 10 : 6) c
     if (lane == 0 && colls) atomicAdd(a.counters + C_COLLISIONS, (unsigned long long)colls);
 }
 
-// Big cells, one at a time by the whole block, giants first: the sliding
-// window of collide_two_cells over 512 threads. The idle threads of a warp
-// take their pairs together from a counter; which of them gets which pair
-// does not matter, only that every pair below a claimed one is claimed or
-// done, and the barrier before the claims are read sees to that.
+// One cell by the whole block: the sliding window of collide_two_cells over
+// kBigThreads threads. The idle threads of a warp take their pairs together
+// from a counter; which of them gets which pair does not matter, only that
+// every pair below a claimed one is claimed or done, and the barrier before
+// the claims are read sees to that. A: the cell's states and claims (an
+// Arena, or InPlace for a cell beyond it).
+template <typename Real, typename States>
+__device__ __forceinline__ void collide_by_block(const States& A, int n, int c, int np, double consCrm, double crm0,
+                                                 const StepArgs<Real>& a, int istep, int* sNext,
+                                                 unsigned long long* sCrm, uint32_t& colls)
+{
+    const int tid = threadIdx.x, lane = tid & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const Real crm0r = (Real)crm0;
+    Real crmLocal = (Real)0;
+    // threads with pairs: more than n / 2 at once mostly wait for each
+    // other and take issue slots from those that go
+    const bool works = tid < min(kBigThreads, max(64, (n >> 1) & ~31));
+    int j = -1, k1 = 0, k2 = 0;
+    uint32_t w2 = 0u, w3 = 0u;
+    bool left = works;  // pairs may be left to hand out (the same in every lane of a warp)
+    // the next pairs to the lanes of this warp that ask for one
+    auto hand_out = [&](bool ask) {
+        const unsigned m = __ballot_sync(kFull, ask);
+        if (ask) j = -1;
+        if (!left || !m) return;
+        int first = 0;
+        if (lane == 0) first = atomicAdd(sNext, __popc(m));
+        first = __shfl_sync(kFull, first, 0);
+        const int jj = first + __popc(m & below);
+        if (ask && jj < np) {
+            j = jj;
+            const PairDraw d = pair_draw(c, istep, j, n, a.C, k1, k2);
+            w2 = d.b0.z;
+            w3 = d.b0.w;
+        }
+        left = first < np;
+    };
+    hand_out(works);
+    for (;;) {
+        if (j >= 0) {
+            atomicMin(&A.claim[k1], j);
+            atomicMin(&A.claim[k2], j);
+        }
+        __syncthreads();
+        const bool go = j >= 0 && A.claim[k1] == j && A.claim[k2] == j;
+        __syncthreads();
+        const int jNow = j, k1Now = k1, k2Now = k2;
+        const uint32_t w2Now = w2, w3Now = w3;
+        hand_out(go);   // drawn beside this round's collisions, claimed in the next
+        if (go) {
+            PState<Real> p = A.get(k1Now), q = A.get(k2Now);
+            if (pair_collide<Real>(p, q, c, istep, jNow, w2Now, w3Now, a.C, consCrm, crm0r, n > kStagedSum, crmLocal)) {
+                A.put(k1Now, p);
+                A.put(k2Now, q);
+                ++colls;
+            }
+            A.claim[k1Now] = INT_MAX;
+            A.claim[k2Now] = INT_MAX;
+        }
+        if (!__syncthreads_or(j >= 0)) break;
+    }
+    // the largest relative speed tested (a double's order is that of
+    // its bits when positive)
+    const double m = largest_speed(warp_max(crmLocal));
+    if (lane == 0 && m > crm0) atomicMax(sCrm, (unsigned long long)__double_as_longlong(m));
+}
+
+// Big cells, one at a time by a block, giants first, then the middle cells if
+// the blocks take them. A cell beyond the block's arena is run in place in
+// the particle buffer, its claims in its cell-id slots.
 template <typename Real>
-__global__ void __launch_bounds__(kBigThreads, 1) collide_big_kernel(StepArgs<Real> a)
+__global__ void __launch_bounds__(kBigThreads, kBigPerSm) collide_big_kernel(StepArgs<Real> a)
 {
     extern __shared__ __align__(16) unsigned char cellSmem[];
     __shared__ int sItem, sNext;
     __shared__ unsigned long long sCrm;
     const int tid = threadIdx.x, lane = tid & 31;
-    const unsigned below = (1u << lane) - 1u;
     const Arena<Real> A(cellSmem, kBigArena);
     const int istep = a.ctl->istep, ncell = a.M.ncell;
     const int nBig = a.cellWork[4], nGiant = a.cellWork[5];
+    const int nAll = nBig + nGiant + (middle_by_blocks(a.cellWork, (int)gridDim.x) ? a.cellWork[9] : 0);
     const PBuf<Real> buf = a.A;
     uint32_t colls = 0;
-    if (nBig + nGiant > 0)
+    if (nAll > 0)
         for (;;) {
             __syncthreads();   // the last cell's values have been read
             if (tid == 0) {
@@ -1724,71 +1806,24 @@ __global__ void __launch_bounds__(kBigThreads, 1) collide_big_kernel(StepArgs<Re
             }
             __syncthreads();
             const int it = sItem;
-            if (it >= nBig + nGiant) break;
-            const int c = a.cellList[it < nGiant ? ncell + it : ncell - 1 - (it - nGiant)];
+            if (it >= nAll) break;
+            const int c = it < nGiant ? a.cellList[ncell + it]
+                          : it < nGiant + nBig ? a.cellList[ncell - 1 - (it - nGiant)]
+                                               : a.cellItem[2 * ncell - 1 - (it - nGiant - nBig)].x;
             const int s0 = a.startA[c], n = a.startA[c + 1] - s0, np = a.cellPairs[c];
             const double consCrm = a.cellCons[c], crm0 = a.crmax[c];
-            if (n > kBigArena) {
-                if (tid < 32) collide_cell_in_place<Real>(buf, s0, n, c, np, consCrm, crm0, a, istep, colls);
-                continue;
-            }
-            stage_cell(buf, A, s0, n, 0, tid, kBigThreads);
-            __syncthreads();
-            const Real crm0r = (Real)crm0;
-            Real crmLocal = (Real)0;
-            // threads with pairs: more than n / 2 at once mostly wait for each
-            // other and take issue slots from those that go
-            const bool works = tid < min(kBigThreads, max(64, (n >> 1) & ~31));
-            int j = -1, k1 = 0, k2 = 0;
-            uint32_t w2 = 0u, w3 = 0u;
-            bool left = works;  // pairs may be left to hand out (the same in every lane of a warp)
-            // the next pairs to the lanes of this warp that ask for one
-            auto hand_out = [&](bool ask) {
-                const unsigned m = __ballot_sync(kFull, ask);
-                if (ask) j = -1;
-                if (!left || !m) return;
-                int first = 0;
-                if (lane == 0) first = atomicAdd(&sNext, __popc(m));
-                first = __shfl_sync(kFull, first, 0);
-                const int jj = first + __popc(m & below);
-                if (ask && jj < np) {
-                    j = jj;
-                    const PairDraw d = pair_draw(c, istep, j, n, a.C, k1, k2);
-                    w2 = d.b0.z;
-                    w3 = d.b0.w;
-                }
-                left = first < np;
-            };
-            hand_out(works);
-            for (;;) {
-                if (j >= 0) {
-                    atomicMin(&A.claim[k1], j);
-                    atomicMin(&A.claim[k2], j);
-                }
+            if (n <= kBigArena) {
+                stage_cell(buf, A, s0, n, 0, tid, kBigThreads);
                 __syncthreads();
-                const bool go = j >= 0 && A.claim[k1] == j && A.claim[k2] == j;
+                collide_by_block<Real>(A, n, c, np, consCrm, crm0, a, istep, &sNext, &sCrm, colls);
+                unstage_cell(buf, A, s0, n, 0, tid, kBigThreads);
+            } else {
+                const InPlace<Real> I{{buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0}, buf.cell + s0};
+                for (int k = tid; k < n; k += kBigThreads) I.claim[k] = INT_MAX;
                 __syncthreads();
-                const int jNow = j, k1Now = k1, k2Now = k2;
-                const uint32_t w2Now = w2, w3Now = w3;
-                hand_out(go);   // drawn beside this round's collisions, claimed in the next
-                if (go) {
-                    PState<Real> p = A.get(k1Now), q = A.get(k2Now);
-                    if (pair_collide<Real>(p, q, c, istep, jNow, w2Now, w3Now, a.C, consCrm, crm0r, n > kArena,
-                                           crmLocal)) {
-                        A.put(k1Now, p);
-                        A.put(k2Now, q);
-                        ++colls;
-                    }
-                    A.claim[k1Now] = INT_MAX;
-                    A.claim[k2Now] = INT_MAX;
-                }
-                if (!__syncthreads_or(j >= 0)) break;
+                collide_by_block<Real>(I, n, c, np, consCrm, crm0, a, istep, &sNext, &sCrm, colls);
+                for (int k = tid; k < n; k += kBigThreads) I.claim[k] = c;
             }
-            // the largest relative speed tested (a double's order is that of
-            // its bits when positive)
-            const double m = largest_speed(warp_max(crmLocal));
-            if (lane == 0 && m > crm0) atomicMax(&sCrm, (unsigned long long)__double_as_longlong(m));
-            unstage_cell(buf, A, s0, n, 0, tid, kBigThreads);
             __syncthreads();
             if (tid == 0 && sCrm) a.crmax[c] = __longlong_as_double((long long)sCrm);
         }
@@ -1808,7 +1843,7 @@ int CellOcc<Real>::blocks = 1;
 template <typename Real>
 cudaError_t prepare_kernels()
 {
-    constexpr size_t cellBytes = kCellWarps * arena_bytes<Real>(kArena), bigBytes = arena_bytes<Real>(kBigArena);
+    constexpr size_t cellBytes = kCellWarps * arena_bytes<Real>(CellShape<Real>::arena), bigBytes = arena_bytes<Real>(kBigArena);
     cudaError_t e = cudaFuncSetAttribute(collide_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cellBytes);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(collide_big_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bigBytes);
@@ -1831,11 +1866,12 @@ void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t 
     // the big cells' kernel goes first: its blocks need much of an SM's
     // shared memory, and the other cells' blocks fill what they leave
     side.fork(s);
-    collide_big_kernel<Real><<<L.smCount, kBigThreads, arena_bytes<Real>(kBigArena), side.stream>>>(a);
+    const int bigBlocks = L.smCount * kBigPerSm;
+    collide_big_kernel<Real><<<bigBlocks, kBigThreads, arena_bytes<Real>(kBigArena), side.stream>>>(a);
     int g = (ncell + kCellWarps - 1) / kCellWarps;
     const int cap = L.smCount * min(CellOcc<Real>::blocks, max(1, L.collideBlocksPerSm));
     if (g > cap) g = cap;
-    collide_kernel<Real><<<g > 0 ? g : 1, kCellWarps * 32, kCellWarps * arena_bytes<Real>(kArena), s>>>(a);
+    collide_kernel<Real><<<g > 0 ? g : 1, kCellWarps * 32, kCellWarps * arena_bytes<Real>(CellShape<Real>::arena), s>>>(a, bigBlocks);
     side.join(s);
 }
 

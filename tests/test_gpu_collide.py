@@ -107,3 +107,69 @@ def test_mixed_cell_classes_conserve(block, pairs):
         d = np.abs(np.bincount(cell, weights=q1) - np.bincount(cell, weights=q0))
         assert np.all(d <= 70 * 16 * 2.0 ** -24 * np.maximum(n, 1)), d.max()
     assert (vg != v.astype(np.float32)).any(1).sum() > 0.5 * len(cell)
+
+
+def test_fp64_cells_at_the_arenas_ends_match_oracle(block):
+    """A warp's FP64 arena (376) and a block's (2,048), a lane's cells (12),
+    as in test_fp64_cell_classes_match_oracle at 9,000 pairs."""
+    raw, dm, _ = block
+    mess = _mess(dm, 9000)
+    counts = [11, 12, 13, 375, 376, 377, 2047, 2048, 2049]
+    rs = np.random.RandomState(8)
+    cell = np.sort(np.repeat(rs.permutation(dm.ncell)[: len(counts)], counts)).astype(np.int32)
+    lo, hi = I.cell_boxes(dm)
+    u, sig, tN = I.freestream(mess)
+    x = lo[cell] + (hi[cell] - lo[cell]) * rs.random_sample((cell.shape[0], 3))
+    v, ir = u + sig * rs.standard_normal(x.shape), -0.5 * tN * np.log(1.0 - rs.random_sample(cell.shape[0]))
+    with make_case(dm, mess, seed=11) as case:
+        case.upload_particles(x, v, ir, cell)
+        case.collisionDSMC()
+        _, vg, irg, cg = case.download_particles()
+        cs = case.cell_state()
+    o = make_oracle(dm, mess, seed=11)
+    o.set_particles(x, v, ir, cell)
+    o.step(0, gpu.STAGE_COLLIDE)
+    _, vo, iro, co = o.particles()
+    assert np.array_equal(cg, co)
+    assert np.array_equal(cs[1], o.cell_state()[1])
+    ok = rel_close(vg, vo, 1e-9, 1e-12).all(1) & rel_close(irg, iro, 1e-9, 1e-12)
+    assert ok.mean() >= 0.97, ok.mean()
+
+
+@pytest.mark.parametrize("precision", [gpu.PRECISION_FP64, gpu.PRECISION_MIXED])
+def test_who_takes_a_cell_does_not_matter(precision):
+    """100 cells of 200 particles and some 700 pairs, and 100 of 10 particles:
+    alone, blocks take the first and half warps the second; among 500 of the
+    one kind and 5,580 of the other, warps and single lanes. The same bits."""
+    raw, dm = I.block_mesh(8)
+    mess = I.block_mess(dm, 20).copy()
+    vol = np.asarray(dm.cells["area"], dtype=float)
+    order = np.argsort(np.abs(vol - np.median(vol)), kind="stable")
+    rs = np.random.RandomState(2)
+    n = np.full(dm.ncell, 10)
+    n[order[:500]] = 200
+    cell = np.repeat(np.arange(dm.ncell), n).astype(np.int32)
+    lo, hi = I.cell_boxes(dm)
+    u, sig, tN = I.freestream(mess)
+    x = lo[cell] + (hi[cell] - lo[cell]) * rs.random_sample((cell.shape[0], 3))
+    v, ir = u + sig * rs.standard_normal(x.shape), -0.5 * tN * np.log(1.0 - rs.random_sample(cell.shape[0]))
+    few = np.zeros(dm.ncell, bool)
+    few[order[:100]] = True
+    few[order[500:600]] = True
+    few = few[cell]
+    only = few & (n[cell] == 200)
+    with make_case(dm, mess, seed=1, precision=precision) as case:
+        case.upload_particles(x[only], v[only], ir[only], cell[only])
+        case.collisionDSMC()
+        mess["Neff"] = float(mess["Neff"]) * 700.0 * 100 / case.counters()["candidate_pairs"]
+    outs = []
+    for keep in (few, np.ones(few.shape, bool)):
+        with make_case(dm, mess, seed=9, precision=precision) as case:
+            case.upload_particles(x[keep], v[keep], ir[keep], cell[keep])
+            case.collisionDSMC()
+            _, vg, irg, _ = case.download_particles()
+            outs.append((vg[few[keep]], irg[few[keep]], case.counters()["candidate_pairs"]))
+    assert 100 * 512 < outs[0][2] < 100 * 1024
+    assert np.array_equal(outs[0][0], outs[1][0])
+    assert np.array_equal(outs[0][1], outs[1][1])
+    assert (outs[0][0] != v[few].astype(outs[0][0].dtype)).any(1).mean() > 0.5
