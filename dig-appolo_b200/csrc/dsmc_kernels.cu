@@ -1288,7 +1288,6 @@ constexpr int kCellWarps = 2;                 // warps per block of collide_kern
 constexpr int kSmallMax = 16;
 constexpr int kBigThreads = 256;
 constexpr int kBigPerSm = 2;                  // resident blocks of collide_big_kernel per SM
-constexpr int kBigArena = 2048;               // staged particles per block of collide_big_kernel
 constexpr int kBigPairs = 1024, kMiddlePairs = 512;
 constexpr int kBigLeast = 128;                // fewer particles give a block no more pairs a round than a warp
 template <typename Real>
@@ -1298,12 +1297,14 @@ struct CellShape<float> {
     static constexpr int arena = 512;         // staged particles per warp
     static constexpr int blocks = 10;         // resident blocks of collide_kernel per SM
     static constexpr int small = kSmallMax;   // particles of a small cell
+    static constexpr int big = 4096;          // staged particles per block of collide_big_kernel
 };
 template <>
 struct CellShape<double> {
     static constexpr int arena = 376;
     static constexpr int blocks = 8;
     static constexpr int small = 12;
+    static constexpr int big = 3072;
 };
 constexpr int kSmallPairs = 32;
 constexpr int kGiantPairs = 8192;
@@ -1782,7 +1783,8 @@ __device__ __forceinline__ void collide_by_block(const States& A, int n, int c, 
 
 // Big cells, one at a time by a block, giants first, then the middle cells if
 // the blocks take them. A cell beyond the block's arena is run in place in
-// the particle buffer, its claims in its cell-id slots.
+// the particle buffer, with its claims in the arena's memory or, beyond that
+// too (20,480 particles in FP32, 27,648 in FP64), in its cell-id slots.
 template <typename Real>
 __global__ void __launch_bounds__(kBigThreads, kBigPerSm) collide_big_kernel(StepArgs<Real> a)
 {
@@ -1790,7 +1792,9 @@ __global__ void __launch_bounds__(kBigThreads, kBigPerSm) collide_big_kernel(Ste
     __shared__ int sItem, sNext;
     __shared__ unsigned long long sCrm;
     const int tid = threadIdx.x, lane = tid & 31;
-    const Arena<Real> A(cellSmem, kBigArena);
+    constexpr int kArena = CellShape<Real>::big;
+    constexpr int kClaims = (int)(arena_bytes<Real>(kArena) / sizeof(int));
+    const Arena<Real> A(cellSmem, kArena);
     const int istep = a.ctl->istep, ncell = a.M.ncell;
     const int nBig = a.cellWork[4], nGiant = a.cellWork[5];
     const int nAll = nBig + nGiant + (middle_by_blocks(a.cellWork, (int)gridDim.x) ? a.cellWork[9] : 0);
@@ -1812,17 +1816,19 @@ __global__ void __launch_bounds__(kBigThreads, kBigPerSm) collide_big_kernel(Ste
                                                : a.cellItem[2 * ncell - 1 - (it - nGiant - nBig)].x;
             const int s0 = a.startA[c], n = a.startA[c + 1] - s0, np = a.cellPairs[c];
             const double consCrm = a.cellCons[c], crm0 = a.crmax[c];
-            if (n <= kBigArena) {
+            if (n <= kArena) {
                 stage_cell(buf, A, s0, n, 0, tid, kBigThreads);
                 __syncthreads();
                 collide_by_block<Real>(A, n, c, np, consCrm, crm0, a, istep, &sNext, &sCrm, colls);
                 unstage_cell(buf, A, s0, n, 0, tid, kBigThreads);
             } else {
-                const InPlace<Real> I{{buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0}, buf.cell + s0};
+                const InPlace<Real> I{{buf.v[0] + s0, buf.v[1] + s0, buf.v[2] + s0, buf.ir + s0},
+                                      n <= kClaims ? reinterpret_cast<int*>(cellSmem) : buf.cell + s0};
                 for (int k = tid; k < n; k += kBigThreads) I.claim[k] = INT_MAX;
                 __syncthreads();
                 collide_by_block<Real>(I, n, c, np, consCrm, crm0, a, istep, &sNext, &sCrm, colls);
-                for (int k = tid; k < n; k += kBigThreads) I.claim[k] = c;
+                if (n > kClaims)
+                    for (int k = tid; k < n; k += kBigThreads) I.claim[k] = c;
             }
             __syncthreads();
             if (tid == 0 && sCrm) a.crmax[c] = __longlong_as_double((long long)sCrm);
@@ -1843,7 +1849,7 @@ int CellOcc<Real>::blocks = 1;
 template <typename Real>
 cudaError_t prepare_kernels()
 {
-    constexpr size_t cellBytes = kCellWarps * arena_bytes<Real>(CellShape<Real>::arena), bigBytes = arena_bytes<Real>(kBigArena);
+    constexpr size_t cellBytes = kCellWarps * arena_bytes<Real>(CellShape<Real>::arena), bigBytes = arena_bytes<Real>(CellShape<Real>::big);
     cudaError_t e = cudaFuncSetAttribute(collide_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cellBytes);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(collide_big_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bigBytes);
@@ -1867,7 +1873,7 @@ void launch_collide(const StepArgs<Real>& a, const LaunchShape& L, cudaStream_t 
     // shared memory, and the other cells' blocks fill what they leave
     side.fork(s);
     const int bigBlocks = L.smCount * kBigPerSm;
-    collide_big_kernel<Real><<<bigBlocks, kBigThreads, arena_bytes<Real>(kBigArena), side.stream>>>(a);
+    collide_big_kernel<Real><<<bigBlocks, kBigThreads, arena_bytes<Real>(CellShape<Real>::big), side.stream>>>(a);
     int g = (ncell + kCellWarps - 1) / kCellWarps;
     const int cap = L.smCount * min(CellOcc<Real>::blocks, max(1, L.collideBlocksPerSm));
     if (g > cap) g = cap;
