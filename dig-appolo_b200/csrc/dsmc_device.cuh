@@ -463,6 +463,9 @@ __device__ __forceinline__ PlaneHit find_exit_planes(const DevMesh& M, int cell,
 // faces, 160 for 6), which a particle entering the cell misses once instead
 // of in three arrays; the planes, the centre (3 doubles), the scale, the
 // kFaces determinants. Else from the mesh's arrays.
+// Read through __ldg: nothing writes it while a kernel runs, and loads that
+// the compiler knows to be constant move ahead of a particle's stores (20,800
+// tetrahedra, the step: 485 -> 481.6 us; 372,500: 4,146 -> 4,132).
 template <int kFaces>
 struct CellGeo {
     static constexpr int kFloats = kFaces == 6 ? 40 : 32;
@@ -471,10 +474,10 @@ struct CellGeo {
         : at(M.geo + (size_t)cell * (kFloats / 4))
     {
     }
-    __device__ __forceinline__ float4 plane(int k) const { return at[k]; }
+    __device__ __forceinline__ float4 plane(int k) const { return __ldg(at + k); }
     __device__ __forceinline__ const double* centre() const { return reinterpret_cast<const double*>(at + kFaces); }
-    __device__ __forceinline__ float scale() const { return reinterpret_cast<const float*>(at + kFaces)[6]; }
-    __device__ __forceinline__ float det(int k) const { return reinterpret_cast<const float*>(at + kFaces)[7 + k]; }
+    __device__ __forceinline__ float scale() const { return __ldg(reinterpret_cast<const float*>(at + kFaces) + 6); }
+    __device__ __forceinline__ float det(int k) const { return __ldg(reinterpret_cast<const float*>(at + kFaces) + 7 + k); }
 };
 template <>
 struct CellGeo<0> {
@@ -596,7 +599,7 @@ __device__ __forceinline__ CertainExit certain_exit_f32(const DevMesh& M, int ce
         r.tLo = bestLo;
         return r;
     }
-    const int4 rec = M.faceRec[b + bi];
+    const int4 rec = __ldg(M.faceRec + b + bi);
     int tri = -1, triIdx = M.triPerRec ? (b + bi) * M.triPerRec : rec.y;
     if ((rec.z & 0xff) == 4) {
         const float4 dg = M.diagF[b + bi];
@@ -644,7 +647,7 @@ __device__ __forceinline__ CertainExit search_certain(const DevMesh& M, int cell
                                                       const PRegs<Real>& p)
 {
     const double* cc = cell_centre<kFaces>(M, cell);
-    const float xr[3] = {(float)ds(p.x[0], cc[0]), (float)ds(p.x[1], cc[1]), (float)ds(p.x[2], cc[2])};
+    const float xr[3] = {(float)ds(p.x[0], __ldg(cc)), (float)ds(p.x[1], __ldg(cc + 1)), (float)ds(p.x[2], __ldg(cc + 2))};
     const float v[3] = {(float)p.v[0], (float)p.v[1], (float)p.v[2]};
     CertainExit ce = certain_exit_f32<kAtRest, kFaces>(M, cell, crossf, entry, tag, xr, v);
     if constexpr (sizeof(Real) == 8) ce.certain = ce.certain && fabsf(v[0]) + fabsf(v[1]) + fabsf(v[2]) > 1e-20f;

@@ -39,9 +39,9 @@ __device__ __forceinline__ void load_position(const DevMesh& M, const PBuf<Real>
         p.x[0] = B.x[0][i]; p.x[1] = B.x[1][i]; p.x[2] = B.x[2][i];
     } else {
         const double* cc = cell_centre<kFaces>(M, cell);
-        p.x[0] = da(cc[0], (double)B.x[0][i]);
-        p.x[1] = da(cc[1], (double)B.x[1][i]);
-        p.x[2] = da(cc[2], (double)B.x[2][i]);
+        p.x[0] = da(__ldg(cc), (double)B.x[0][i]);
+        p.x[1] = da(__ldg(cc + 1), (double)B.x[1][i]);
+        p.x[2] = da(__ldg(cc + 2), (double)B.x[2][i]);
     }
 }
 
@@ -54,9 +54,9 @@ __device__ __forceinline__ void store_position(const DevMesh& M, const PBuf<Real
     } else {
         if (cell < 0 || cell >= M.ncell) return;   // removed: the slot is not read again
         const double* cc = cell_centre<kFaces>(M, cell);
-        B.x[0][i] = (float)ds(p.x[0], cc[0]);
-        B.x[1][i] = (float)ds(p.x[1], cc[1]);
-        B.x[2][i] = (float)ds(p.x[2], cc[2]);
+        B.x[0][i] = (float)ds(p.x[0], __ldg(cc + 0));
+        B.x[1][i] = (float)ds(p.x[1], __ldg(cc + 1));
+        B.x[2][i] = (float)ds(p.x[2], __ldg(cc + 2));
     }
 }
 
@@ -377,9 +377,9 @@ __global__ void __launch_bounds__(256) move_stay_kernel(StepArgs<Real> a)
                     p[k].x[0] = xs[k][0]; p[k].x[1] = xs[k][1]; p[k].x[2] = xs[k][2];
                 } else {
                     const double* cc = cell_centre<kFaces>(a.M, cell[k]);
-                    p[k].x[0] = da(cc[0], (double)xs[k][0]);
-                    p[k].x[1] = da(cc[1], (double)xs[k][1]);
-                    p[k].x[2] = da(cc[2], (double)xs[k][2]);
+                    p[k].x[0] = da(__ldg(cc + 0), (double)xs[k][0]);
+                    p[k].x[1] = da(__ldg(cc + 1), (double)xs[k][1]);
+                    p[k].x[2] = da(__ldg(cc + 2), (double)xs[k][2]);
                 }
                 if (stays_for_the_step<Real, kFaces>(a.M, cell[k], xs[k], p[k], dt)) {
                     advance(p[k], dt);
