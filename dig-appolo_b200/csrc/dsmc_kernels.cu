@@ -2374,7 +2374,9 @@ __global__ void download_widen_kernel(const float* __restrict__ in, const int* _
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double v = (double)in[i];
-        if (comp < 3) v = da(center[(size_t)cell[i] * 3 + comp], v);
+        // a slot whose particle the move removed (cell -1, before the sort)
+        // has no centre
+        if (comp < 3 && cell[i] >= 0) v = da(center[(size_t)cell[i] * 3 + comp], v);
         out[i] = v;
     }
 }

@@ -41,6 +41,24 @@ def test_upload_download_round_trip(block, n, precision):
             assert np.array_equal(irg, f32(ir[want]) if mixed else ir[want])
 
 
+@pytest.mark.parametrize("precision", [gpu.PRECISION_FP64, gpu.PRECISION_MIXED])
+def test_download_between_move_and_sort(block, precision):
+    """Slots of removed particles (cell -1) are still there; every other
+    particle lies in its cell, to the rounding of an FP32 offset."""
+    raw, dm, mess = block
+    x, v, ir, cell = _particles(dm, mess, 70000, 3)
+    lo, hi = I.cell_boxes(dm)
+    with make_case(dm, mess, precision=precision) as case:
+        case.upload_particles(x, v, ir, cell)
+        case.advection(1)
+        xg, vg, irg, cg = case.download_particles()
+        cnt = case.counters()
+    removed = cnt["removed"] + cnt["dropped"] + cnt["lost"]
+    live = cg >= 0
+    assert removed > 0 and (~live).sum() == removed
+    assert np.all(xg[live] >= lo[cg[live]] - 1e-6) and np.all(xg[live] <= hi[cg[live]] + 1e-6)
+
+
 @pytest.mark.parametrize("n", [65537, 131072, 131075])
 def test_trace_in_chunks_matches_oracle(block, n):
     """With wall re-emission, whose random streams are numbered by particle:
