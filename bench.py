@@ -551,8 +551,8 @@ def gsis_timing(case, wl, seed: int, repeats: int = 3) -> dict:
 def launches_per_step(wl) -> int:
     # inject: count, scan, generate; move: stay pass, tracing pass; sort:
     # rank, scan x2, scatter, far-slot order, gather; collide: classify,
-    # collide; sample
-    return 3 + 2 + 6 + 2 + 1
+    # big cells, the others; sample
+    return 3 + 2 + 6 + 3 + 1
 
 
 def run_e2e_k(wl, plan, args, init, shape, rank):
