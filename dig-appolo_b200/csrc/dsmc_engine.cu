@@ -178,7 +178,8 @@ struct Engine {
     double stageMs[5] = {0, 0, 0, 0, 0};
     int64_t timedSteps = 0;
     HostLink link;                 // pageable host arrays to and from the device
-    char* traceWork = nullptr;     // dsmc_trace's device memory, for kTraceChunk particles at a time
+    char* traceWork = nullptr;     // dsmc_trace's device memory, for traceRoom particles at a time
+    int64_t traceRoom = 0;
 
     ~Engine() { release(); }
 
@@ -190,6 +191,7 @@ struct Engine {
         for (auto& e : ev)
             if (e) { cudaEventDestroy(e); e = nullptr; }
         link.release();
+        if (traceWork) { cudaFree(traceWork); traceWork = nullptr; traceRoom = 0; }
         for (void* p : allocs) cudaFree(p);
         allocs.clear();
         if (side.forked) { cudaEventDestroy(side.forked); side.forked = nullptr; }
@@ -840,6 +842,7 @@ struct Engine {
             !alloc(cellItem, (size_t)ncell * 2) || !alloc(cellItemC, (size_t)ncell * 2) ||
             !alloc(errorWord, 1) || !alloc(uploadFlag, 1))
             return false;
+        if (precision == DSMC_PRECISION_MIXED && !alloc(link.staged, HostLink::kSlots * HostLink::kBytes, false)) return false;
         if (params.keep_step_moments && !alloc(stepMom, (size_t)ncell * 18)) return false;
         cudaError_t pe = (precision == DSMC_PRECISION_MIXED) ? prepare_kernels<float>() : prepare_kernels<double>();
         if (!cuda(pe, "kernel attributes")) return false;
@@ -1731,18 +1734,31 @@ struct Engine {
         return true;
     }
 
-    // The tracing check in chunks of kTraceChunk particles, so that its device
-    // memory (19 MB, kept on the handle from the first call) does not grow
-    // with n; the conversions between FP64 and the working precision run on
-    // the device.
+    // The tracing check in chunks of kTraceChunk particles. Its device memory
+    // (140 bytes a particle of the largest call, at most a chunk's 18 MB) stays
+    // on the handle; the conversions between FP64 and the working precision run
+    // on the device.
     static constexpr int64_t kTraceChunk = 1 << 17;
     bool trace(int64_t n, const double* const src[7], const int32_t* cell, int stopAtWall, int32_t* const iout[5],
                double* const fout[7])
     {
         const bool mixed = precision == DSMC_PRECISION_MIXED;
-        const size_t N = (size_t)kTraceChunk;
-        // six FP64 columns and dt each way, the cells, six result columns
-        if (!traceWork && !alloc(traceWork, N * (14 * 8 + 7 * 4), false)) return false;
+        // six FP64 columns and dt each way, the cells, six result columns, for
+        // as many particles as a chunk of the largest call so far
+        const int64_t room = std::min(n, kTraceChunk);
+        if (room > traceRoom) {
+            if (traceWork) cudaFree(traceWork);
+            traceWork = nullptr;
+            traceRoom = 0;
+            void* q = nullptr;
+            if (cudaMalloc(&q, (size_t)room * (14 * 8 + 7 * 4)) != cudaSuccess) {
+                (void)cudaGetLastError();   // reported here, not by a later launch
+                return fail("trace: device allocation failed (cudaMalloc)");
+            }
+            traceWork = static_cast<char*>(q);
+            traceRoom = room;
+        }
+        const size_t N = (size_t)traceRoom;
         if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
         double* dIn = reinterpret_cast<double*>(traceWork);
         double* dOut = dIn + 7 * N;

@@ -7,12 +7,15 @@
 // the other. What a block's values become on the way, a conversion on the
 // device or a gather on the host, is the caller's. The pinned memory, 6 MB,
 // is allocated on the first use and freed with the handle: the two 64 MB
-// blocks that uploads passed through before took 90 ms to pin.
+// blocks that uploads passed through before took 90 ms to pin. Where none can
+// be pinned, ordinary memory does (the copies then wait). A transfer
+// allocates no device memory.
 #pragma once
 
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstdlib>
 #include <cuda_runtime.h>
 #include <thread>
 
@@ -27,7 +30,8 @@ struct HostLink {
     int device = 0;
     cudaStream_t stream = nullptr;
     char* pinned = nullptr;          // [kSlots][kBytes]
-    char* staged = nullptr;          // the same on the device, for values converted there
+    char* pageable = nullptr;        // ordinary memory instead, or nullptr
+    char* staged = nullptr;          // the same on the device, for values converted there (the caller's)
     cudaEvent_t event[kSlots] = {};
 
     // A block of column `col`: values [off, off + len), with its memory.
@@ -43,8 +47,11 @@ struct HostLink {
         device = dev;
         stream = s;
         cudaError_t e = cudaSuccess;
-        if (!pinned) e = cudaHostAlloc((void**)&pinned, kSlots * kBytes, cudaHostAllocDefault);
-        if (e == cudaSuccess && !staged) e = cudaMalloc((void**)&staged, kSlots * kBytes);
+        if (!pinned && cudaHostAlloc((void**)&pinned, kSlots * kBytes, cudaHostAllocDefault) != cudaSuccess) {
+            (void)cudaGetLastError();
+            pinned = pageable = static_cast<char*>(std::malloc(kSlots * kBytes));
+            if (!pinned) return cudaErrorMemoryAllocation;
+        }
         for (cudaEvent_t& ev : event)
             if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (e != cudaSuccess) (void)cudaGetLastError();   // reported here, not by a later launch
@@ -54,8 +61,9 @@ struct HostLink {
     {
         for (cudaEvent_t& ev : event)
             if (ev) { cudaEventDestroy(ev); ev = nullptr; }
-        if (staged) { cudaFree(staged); staged = nullptr; }
-        if (pinned) { cudaFreeHost(pinned); pinned = nullptr; }
+        if (pageable) std::free(pageable);
+        else if (pinned) cudaFreeHost(pinned);
+        pinned = pageable = nullptr;
     }
 
     // Host to device. fill(block) writes the block's values to block.host;

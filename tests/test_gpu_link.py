@@ -72,3 +72,17 @@ def test_trace_in_chunks_matches_oracle(block, n):
         assert np.array_equal(g[k], o[k]), k
     for k in ("x", "v", "dt"):
         assert np.all(rel_close(g[k], o[k], 1e-9, 1e-12)), k
+
+
+def test_trace_memory_grows(block):
+    """A small call, a larger one and the small one again, on one handle,
+    against fresh handles."""
+    raw, dm, mess = block
+    x, v, dt, cell = I.trace_inputs(dm, mess, 70001, 6)
+    with make_case(dm, mess, seed=5, precision=gpu.PRECISION_MIXED) as case:
+        kept = [case.trace(x[:n], v[:n], dt[:n], cell[:n], stop_at_wall=False) for n in (33, 70001, 33)]
+    for n, g in zip((33, 70001, 33), kept):
+        with make_case(dm, mess, seed=5, precision=gpu.PRECISION_MIXED) as case:
+            f = case.trace(x[:n], v[:n], dt[:n], cell[:n], stop_at_wall=False)
+        for k in f:
+            assert np.array_equal(f[k], g[k]), k
