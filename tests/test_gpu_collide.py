@@ -173,3 +173,42 @@ def test_who_takes_a_cell_does_not_matter(precision):
     assert np.array_equal(outs[0][0], outs[1][0])
     assert np.array_equal(outs[0][1], outs[1][1])
     assert (outs[0][0] != v[few].astype(outs[0][0].dtype)).any(1).mean() > 0.5
+
+
+@pytest.mark.parametrize("precision", [gpu.PRECISION_FP64, gpu.PRECISION_MIXED])
+def test_cells_beyond_a_blocks_arena(block, precision):
+    """Cells run in place: at the end of a block's arena (3,072 in FP64, 4,096
+    in FP32) and of the claims that fit its memory (27,648 and 20,480), with
+    3.4 pairs a particle at most. FP64 against the oracle as in
+    test_fp64_cell_classes_match_oracle; mixed keeps every cell's momentum and
+    energy to the bound of test_mixed_cell_classes_conserve. The claims leave
+    no trace in the cell ids."""
+    raw, dm, _ = block
+    mess = _mess(dm, 1000)
+    counts = [3072, 3073, 27648, 27649] if precision == gpu.PRECISION_FP64 else [4096, 4097, 20480, 20481]
+    rs = np.random.RandomState(8)
+    cell = np.sort(np.repeat(rs.permutation(dm.ncell)[: len(counts)], counts)).astype(np.int32)
+    lo, hi = I.cell_boxes(dm)
+    u, sig, tN = I.freestream(mess)
+    x = lo[cell] + (hi[cell] - lo[cell]) * rs.random_sample((cell.shape[0], 3))
+    v, ir = u + sig * rs.standard_normal(x.shape), -0.5 * tN * np.log(1.0 - rs.random_sample(cell.shape[0]))
+    with make_case(dm, mess, seed=11, precision=precision) as case:
+        case.upload_particles(x, v, ir, cell)
+        case.collisionDSMC()
+        _, vg, irg, cg = case.download_particles()
+        cnt = case.counters()
+    assert np.array_equal(cg, cell)
+    assert cnt["collisions"] > 0.05 * len(cell)
+    if precision == gpu.PRECISION_FP64:
+        o = make_oracle(dm, mess, seed=11)
+        o.set_particles(x, v, ir, cell)
+        o.step(0, gpu.STAGE_COLLIDE)
+        _, vo, iro, co = o.particles()
+        assert np.array_equal(co, cell)
+        ok = rel_close(vg, vo, 1e-9, 1e-12).all(1) & rel_close(irg, iro, 1e-9, 1e-12)
+        assert ok.mean() >= 0.97, ok.mean()
+    e0, e1 = 0.5 * (v ** 2).sum(1) + ir, 0.5 * (vg ** 2).sum(1) + irg
+    n = np.bincount(cell)
+    for q0, q1 in ((v[:, 0], vg[:, 0]), (v[:, 1], vg[:, 1]), (v[:, 2], vg[:, 2]), (e0, e1)):
+        d = np.abs(np.bincount(cell, weights=q1) - np.bincount(cell, weights=q0))
+        assert np.all(d <= 70 * 16 * 2.0 ** -24 * np.maximum(n, 1)), d.max()
