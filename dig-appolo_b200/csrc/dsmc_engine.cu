@@ -430,6 +430,8 @@ struct Engine {
             !cuda(cudaEventCreateWithFlags(&side.forked, cudaEventDisableTiming), "cudaEventCreate") ||
             !cuda(cudaEventCreateWithFlags(&side.joined, cudaEventDisableTiming), "cudaEventCreate"))
             return false;
+        link.device = device;
+        link.stream = stream;
         ncell = md->ncell;
         nface = md->nface;
         npoint = md->npoint;
@@ -1346,7 +1348,6 @@ struct Engine {
     int uploadCellMajor(int64_t n, const double* const src[7], const int32_t* cell)
     {
         int* dCell = static_cast<int*>(buf[cur][7]);
-        if (!cuda(link.ensure(device, stream), "pinned staging")) return -1;
         if (hostPinned(cell)) {
             if (!cuda(cudaMemcpyAsync(dCell, cell, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, stream), "upload")) return -1;
         } else if (!cuda(link.in(1, &n,
@@ -1442,7 +1443,6 @@ struct Engine {
         haveParticles = false;
         if (!ensureCapacity(need)) return false;
         const bool mixed = precision == DSMC_PRECISION_MIXED;
-        if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
         // the seven columns and the cell ids, gathered block by block
         int64_t len[8];
         std::fill(len, len + 8, n);
@@ -1696,7 +1696,6 @@ struct Engine {
         if (n == 0) return true;
         double* dst[7] = {px, py, pz, vx, vy, vz, ir};
         const bool mixed = precision == DSMC_PRECISION_MIXED;
-        if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
         int col[8], ncol = 0;
         int64_t len[8];
         for (int k = 0; k < 8; ++k)
@@ -1759,7 +1758,6 @@ struct Engine {
             traceRoom = room;
         }
         const size_t N = (size_t)traceRoom;
-        if (!cuda(link.ensure(device, stream), "pinned staging")) return false;
         double* dIn = reinterpret_cast<double*>(traceWork);
         double* dOut = dIn + 7 * N;
         int* dCell = reinterpret_cast<int*>(dOut + 7 * N);

@@ -1,15 +1,25 @@
 // Columns between pageable host arrays and the device, through a few small
-// pinned blocks (dsmc_upload_particles, dsmc_download_particles, dsmc_trace).
+// blocks of host memory (dsmc_upload_particles, dsmc_download_particles,
+// dsmc_trace).
 //
 // A transfer is cut into blocks of kItems values, taken by up to kThreads
-// host threads; each thread has two pinned blocks, so that the host copy (and
-// with it the page faults of a fresh array) of one overlaps the transfer of
-// the other. What a block's values become on the way, a conversion on the
-// device or a gather on the host, is the caller's. The pinned memory, 6 MB,
-// is allocated on the first use and freed with the handle: the two 64 MB
-// blocks that uploads passed through before took 90 ms to pin. Where none can
-// be pinned, ordinary memory does (the copies then wait). A transfer
-// allocates no device memory.
+// host threads; each thread has two blocks of memory, so that the host copy
+// (and with it the page faults of a fresh array) of one overlaps the transfer
+// of the other. What a block's values become on the way, a conversion on the
+// device or a gather on the host, is the caller's. A transfer allocates no
+// device memory.
+//
+// The blocks, 6 MB, are freed with the handle. They are ordinary memory for
+// the first kPlain bytes that a handle moves and page-locked after that, since
+// page-locking them takes 2.6 to 7.5 ms: a handle that moves little (a few
+// tracing checks, a small restart) does without, and one that moves more has
+// by then gained about as much over the transfers it replaces. First tracing
+// check on a handle, 5,000 / 50,000 / 200,000 particles on 6,080 cells: 0.6 / 3.1 /
+// 9.6 ms (page-locked at once 8.3 / 9.2 / 13.4; a copy per column and array
+// 1.3 / 4.0 / 14.3), later ones 0.3 / 1.4 / 4.8. With kPlain at 16 MB, checks of
+// 50,000 were behind the copies by column until the sixth. Where none can be
+// page-locked, ordinary memory does for good (the copies then wait for each
+// other).
 #pragma once
 
 #include <algorithm>
@@ -27,10 +37,13 @@ struct HostLink {
     static constexpr int64_t kItems = 65536;
     static constexpr size_t kBytes = (size_t)kItems * 8;   // of a block: values of at most 8 bytes
 
-    int device = 0;
+    static constexpr int64_t kPlain = 32 << 20;
+
+    int device = 0;                  // set by the owner
     cudaStream_t stream = nullptr;
-    char* pinned = nullptr;          // [kSlots][kBytes]
-    char* pageable = nullptr;        // ordinary memory instead, or nullptr
+    char* blocks = nullptr;          // [kSlots][kBytes]
+    bool pinned = false;             // whether they are page-locked
+    int64_t plainLeft = kPlain;      // bytes still to be moved through ordinary memory
     char* staged = nullptr;          // the same on the device, for values converted there (the caller's)
     cudaEvent_t event[kSlots] = {};
 
@@ -42,16 +55,24 @@ struct HostLink {
         char* dev;
     };
 
-    cudaError_t ensure(int dev, cudaStream_t s)
+    // Makes the blocks ready for a transfer of `bytes`.
+    cudaError_t ready(int64_t bytes)
     {
-        device = dev;
-        stream = s;
-        cudaError_t e = cudaSuccess;
-        if (!pinned && cudaHostAlloc((void**)&pinned, kSlots * kBytes, cudaHostAllocDefault) != cudaSuccess) {
-            (void)cudaGetLastError();
-            pinned = pageable = static_cast<char*>(std::malloc(kSlots * kBytes));
-            if (!pinned) return cudaErrorMemoryAllocation;
+        if (bytes <= plainLeft) {
+            plainLeft -= bytes;
+        } else if (!pinned && plainLeft >= 0) {
+            plainLeft = -1;
+            void* q = nullptr;
+            if (cudaHostAlloc(&q, kSlots * kBytes, cudaHostAllocDefault) == cudaSuccess) {
+                freeBlocks();
+                blocks = static_cast<char*>(q);
+                pinned = true;
+            } else {
+                (void)cudaGetLastError();
+            }
         }
+        if (!blocks && !(blocks = static_cast<char*>(std::malloc(kSlots * kBytes)))) return cudaErrorMemoryAllocation;
+        cudaError_t e = cudaSuccess;
         for (cudaEvent_t& ev : event)
             if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
         if (e != cudaSuccess) (void)cudaGetLastError();   // reported here, not by a later launch
@@ -59,11 +80,9 @@ struct HostLink {
     }
     void release()
     {
+        freeBlocks();
         for (cudaEvent_t& ev : event)
             if (ev) { cudaEventDestroy(ev); ev = nullptr; }
-        if (pageable) std::free(pageable);
-        else if (pinned) cudaFreeHost(pinned);
-        pinned = pageable = nullptr;
     }
 
     // Host to device. fill(block) writes the block's values to block.host;
@@ -107,6 +126,16 @@ struct HostLink {
     }
 
 private:
+    void freeBlocks()
+    {
+        for (cudaEvent_t ev : event)
+            if (ev) cudaEventSynchronize(ev);   // the copies that read or write them
+        if (pinned) cudaFreeHost(blocks);
+        else std::free(blocks);
+        blocks = nullptr;
+        pinned = false;
+    }
+
     // step(slot, block) for every block, a thread's two slots in turn, and at
     // the end step(slot, nullptr) for each of them, the older first.
     template <class Step>
@@ -117,6 +146,8 @@ private:
             total += (n[c] + kItems - 1) / kItems;
             items += n[c];
         }
+        if (total == 0) return cudaSuccess;
+        if (const cudaError_t e = ready(items * 8)) return e;
         std::atomic<int64_t> next{0};
         std::atomic<int> error{0};
         auto work = [&](int t) {
@@ -130,7 +161,7 @@ private:
                 k.off = q * kItems;
                 k.len = std::min(kItems, n[k.col] - k.off);
                 const int slot = 2 * t + b;
-                k.host = pinned + (size_t)slot * kBytes;
+                k.host = blocks + (size_t)slot * kBytes;
                 k.dev = staged + (size_t)slot * kBytes;
                 e = step(slot, &k);
             }

@@ -1,0 +1,55 @@
+// The few CUDA runtime calls of csrc/dsmc_hostlink.h on the host, counted, for
+// a CPU test of it: copies are done when they are issued, page-locked memory
+// is ordinary memory, and its allocation can be made to fail.
+#pragma once
+
+#include <atomic>
+#include <cstddef>
+#include <cstdlib>
+#include <cstring>
+
+enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2 };
+typedef struct FakeStream* cudaStream_t;
+typedef struct FakeEvent* cudaEvent_t;
+enum { cudaHostAllocDefault = 0, cudaEventDisableTiming = 2 };
+
+namespace fake {
+inline bool failHostAlloc = false;
+inline std::atomic<int> hostAllocs{0}, hostFrees{0}, events{0};
+inline cudaError_t lastError = cudaSuccess;
+}  // namespace fake
+
+inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+inline cudaError_t cudaGetLastError()
+{
+    const cudaError_t e = fake::lastError;
+    fake::lastError = cudaSuccess;
+    return e;
+}
+inline cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
+{
+    if (fake::failHostAlloc) return fake::lastError = cudaErrorMemoryAllocation;
+    ++fake::hostAllocs;
+    *p = std::malloc(n);
+    return cudaSuccess;
+}
+inline cudaError_t cudaFreeHost(void* p)
+{
+    ++fake::hostFrees;
+    std::free(p);
+    return cudaSuccess;
+}
+inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
+{
+    *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));
+    ++fake::events;
+    return cudaSuccess;
+}
+inline cudaError_t cudaEventDestroy(cudaEvent_t e)
+{
+    std::free(e);
+    --fake::events;
+    return cudaSuccess;
+}
+inline cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return e ? cudaSuccess : cudaErrorInvalidValue; }
+inline cudaError_t cudaEventSynchronize(cudaEvent_t e) { return e ? cudaSuccess : cudaErrorInvalidValue; }
