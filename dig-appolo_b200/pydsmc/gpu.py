@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
-from concurrent.futures import ThreadPoolExecutor
+import threading
 
 import numpy as np
 
@@ -173,25 +173,33 @@ def _ptr(a):
     return None if a is None else a.ctypes.data_as(C.c_void_p)
 
 
-_rows_pool = None
-
-
 def _rows(cols):
     """np.stack(cols, 1), by several threads for long columns (the strided
-    copy and the page faults of the new array are most of a download)."""
-    global _rows_pool
+    copy and the page faults of the new array are most of a download). The
+    threads are the call's own: a pool kept between calls takes no work once
+    the interpreter has begun to exit."""
     n = cols[0].shape[0]
     if n < 1 << 16:
         return np.stack(cols, 1)
-    if _rows_pool is None:
-        _rows_pool = ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1)))
     out = np.empty((n, len(cols)), dtype=cols[0].dtype)
+    parts = iter(range(0, n, 1 << 16))
 
-    def part(a):
-        for k, c in enumerate(cols):
-            out[a:a + (1 << 16), k] = c[a:a + (1 << 16)]
+    def work():
+        for a in parts:
+            for k, c in enumerate(cols):
+                out[a:a + (1 << 16), k] = c[a:a + (1 << 16)]
 
-    list(_rows_pool.map(part, range(0, n, 1 << 16)))
+    threads = []
+    try:
+        for _ in range(min(8, os.cpu_count() or 1, -(-n >> 16)) - 1):
+            t = threading.Thread(target=work)
+            t.start()
+            threads.append(t)
+    except RuntimeError:      # no thread to be had (a limit, the interpreter's exit): the others take its parts
+        pass
+    work()
+    for t in threads:
+        t.join()
     return out
 
 
