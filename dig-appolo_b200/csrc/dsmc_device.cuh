@@ -94,6 +94,9 @@ struct DevMesh {
     const double* placeVol;      // [nplace]
 };
 
+// largest |1 - 2 eta| for which FP32 settles FP64 acceptances (pair_accept)
+constexpr float kVhsSettled = 8.0f;
+
 struct DevConsts {
     double dtime;
     double twall;        // Twall_ref
@@ -106,6 +109,7 @@ struct DevConsts {
     double expLB;        // 1 / (2.5 - omega): Larsen-Borgnakke energy-fraction exponent
     double invAlpha;     // 1 / alpha: VSS scattering exponent
     float vhsExpF;       // 1 - 2 eta: exponent of the VHS sigma*c ratio (FP32 path)
+    float vhsHalfF;      // half of it where the FP64 acceptance may be settled in FP32, else NaN (pair_accept)
     float prelaxF;       // P_relax (FP32 path)
     float invPrelaxF;    // 1 / P_relax, 0 when P_relax is 0 (FP32 path)
     uint32_t seedLo, seedHi;

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <new>
 #include <numeric>
@@ -765,6 +766,7 @@ struct Engine {
         C.omega = mess.omega;
         C.eta = mess.eta;
         C.vhsExpF = (float)(1.0 - 2.0 * mess.eta);
+        C.vhsHalfF = std::fabs(C.vhsExpF) <= kVhsSettled ? 0.5f * C.vhsExpF : std::numeric_limits<float>::quiet_NaN();
         C.expLB = 1.0 / (2.5 - mess.omega);
         C.invAlpha = 1.0 / mess.alpha;
         C.prelaxF = (float)mess.P_relax;

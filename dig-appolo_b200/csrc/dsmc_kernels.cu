@@ -1054,15 +1054,22 @@ __device__ __forceinline__ bool pair_accept(const PState<Real>& p, const PState<
         const double cr2 = da(da(dm(vr0, vr0), dm(vr1, vr1)), dm(vr2, vr2));
         speed = cr2;
         const double u = unit64(w2, w3);
-        // The acceptance is (cr / crmax)^(1 - 2 eta). In FP32 it comes out
-        // within 3e-6 of itself for ratios of 2^-60 to 2^60 (the logarithm's
-        // error times its exponent); a variate further than 2^-13 of it away
-        // is settled, and only the others (1 in 10^4) need the square root,
-        // the power and the division of the FP64 test.
+        // The acceptance is (cr / crmax)^e with e = 1 - 2 eta. In FP32, for a
+        // squared ratio r of 2^-60 to 2^60, its exponent (e / 2) log2 r is off
+        // by |e| / 2 times the errors of log2 r, 2^-17 (2 ulp, its documented
+        // bound there) and 2^-20.5 (the roundings of cr2, c0, c0^2 and the
+        // quotient's 2 ulp, times log2(e)), and by |e| 2^-18 (the roundings of e
+        // and of the product): 8e-6 |e|, and the acceptance with exp2f's 2 ulp
+        // by 6e-6 |e| + 3e-7 of itself. At |e| <= kVhsSettled that is 5e-5, under
+        // half of 2^-13: a variate further than 2^-13 of the estimate away is
+        // settled, and only the others (1 in 10^4) need the square root, the
+        // power and the division of the FP64 test. Beyond it (vhsHalfF is NaN)
+        // nothing is settled here. Squares that leave the normal range are
+        // flushed to 0 or are infinite, and r is then out of its range.
         const float c0 = (float)crm0;
         const float r = __fdividef((float)cr2, c0 * c0);
         if (r > 0x1p-60f && r < 0x1p60f) {
-            const float est = exp2f(0.5f * C.vhsExpF * __log2f(r)), uf = (float)u;
+            const float est = exp2f(C.vhsHalfF * __log2f(r)), uf = (float)u;
             if (uf < est * (1.0f - 0x1p-13f)) return true;
             if (uf > est * (1.0f + 0x1p-13f)) return false;
         }
@@ -1070,8 +1077,12 @@ __device__ __forceinline__ bool pair_accept(const PState<Real>& p, const PState<
         return u < accept;
     } else {
         const float vr0 = p.x - q.x, vr1 = p.y - q.y, vr2 = p.z - q.z;
-        // the squares added in one rounding each; in cells whose pairs ran
-        // in place or alone (splitSum) the last one is rounded on its own
+        // the squares added in one rounding each; in cells of up to kSmallMax
+        // or more than kStagedSum particles (splitSum) the last one is rounded on
+        // its own. Neither is the better one: mixed runs have always summed
+        // so (by one lane and in place the one way, staged the other), and one
+        // rounding changed changes every later pair of the run, so which it is
+        // goes by the particle count and not by who runs the cell.
         const float xy = fmaf(vr0, vr0, __fmul_rn(vr1, vr1));
         const float cr = psqrt(splitSum ? __fadd_rn(xy, __fmul_rn(vr2, vr2)) : fmaf(vr2, vr2, xy));
         speed = cr;
