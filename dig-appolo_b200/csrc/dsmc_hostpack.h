@@ -1,6 +1,8 @@
-// Host-side loops of the particle upload and download (dsmc_upload_particles,
-// dsmc_download_particles), split over threads for large particle counts.
-// Plain C++17, no CUDA: the same header builds into a CPU test.
+// Host-side loops of particle uploads in other orders than the library's
+// (dsmc_upload_particles), split over threads for large particle counts; the
+// gathers are called block by block from the transfer's threads
+// (dsmc_hostlink.h). Plain C++17, no CUDA: the same header builds into a CPU
+// test.
 //
 // The order is the library's canonical one: cell-major, and within a cell
 // the input order (a stable counting sort by cell). Conversions are the
@@ -11,7 +13,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
-#include <cstring>
 #include <thread>
 #include <vector>
 
@@ -126,7 +127,9 @@ inline void gather_cells(int64_t n, const int64_t* order, const int32_t* cell, i
     });
 }
 
-// dst[j] = shift[cell[j] * 3 + comp] + (double)src[j]; no shift when shift is null.
+// dst[j] = shift[cell[j] * 3 + comp] + (double)src[j]; no shift when shift is
+// null. The widening of a download on the host: the statement in plain C++ of
+// what download_widen_kernel does on the device.
 template <class In>
 void widen(int64_t n, const In* src, const int32_t* cell, const double* shift, int comp, double* dst, int nthreads)
 {
@@ -136,17 +139,6 @@ void widen(int64_t n, const In* src, const int32_t* cell, const double* shift, i
             if (shift) v = shift[(size_t)cell[j] * 3 + comp] + v;
             dst[j] = v;
         }
-    });
-}
-
-// memcpy split over threads (byte ranges; every thread count gives the same
-// bytes)
-inline void parallel_copy(void* dst, const void* src, size_t bytes, int nthreads)
-{
-    char* d = static_cast<char*>(dst);
-    const char* s = static_cast<const char*>(src);
-    parallel_for((int64_t)bytes, nthreads, [&](int64_t b, int64_t e, int) {
-        if (e > b) std::memcpy(d + b, s + b, (size_t)(e - b));
     });
 }
 

@@ -987,11 +987,6 @@ __device__ __forceinline__ double collision_diameter(double cr, double prefactor
     return dm(dm(cr, prefactor), pow(dd(1.0, cr2), eta));
 }
 
-// Division: IEEE in FP64 (the oracle's rounding), the fast reciprocal form
-// in the FP32 path (operands here are far from the range limits).
-__device__ __forceinline__ double qdiv(double x, double y) { return x / y; }
-__device__ __forceinline__ float qdiv(float x, float y) { return __fdividef(x, y); }
-
 // The random words of candidate pair j of cell c at step istep: Philox
 // blocks n = 0, 1, ... of counter (c, istep, kPurposeCollide | j << 4),
 // read in order as one stream. Block 0 is drawn when the pair is handed out
