@@ -1214,10 +1214,12 @@ struct Engine {
     // The autotuner: runs full steps of this case from step `istep` on,
     // timing each stage with events, and keeps per stage the fastest of a
     // few launch shapes (move: block size x blocks per SM, particles per
-    // thread of the stay pass; rank / scatter / gather: blocks per SM).
-    // Since no kernel's
-    // result depends on its launch shape, the steps it runs are ordinary
-    // steps of the case; on return `istep` is the next step to run.
+    // thread of the stay pass; scatter / gather: blocks per SM, which the rank
+    // pass follows up to 5). Timed steps run the stages one after another, so
+    // the move is timed without the injection beside it.
+    // Since no kernel's result depends on its launch shape, the steps it runs
+    // are ordinary steps of the case; on return `istep` is the next step to
+    // run.
     bool autotune(int& istep, int trialSteps)
     {
         if (trialSteps < 1) return fail("autotune: trial_steps < 1");

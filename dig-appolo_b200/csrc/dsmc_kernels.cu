@@ -2125,9 +2125,9 @@ __device__ __forceinline__ void moment_terms(double x, double y, double z, doubl
 // FP64 addition per particle, and folds it into the cell's accumulators; then
 // lane g finishes cell g, so that the states of all cells of the run are read
 // together. The next particles are loaded while a chain runs. One thread per
-// cell, the same sums took 2 to 2.3 times as long (uncoalesced loads, cells of
-// unlike size in a warp: 63,517 tetrahedra at 100 a cell 473 -> 228 us, 48,640
-// hexahedra at 50 129 -> 55 us).
+// cell, the same sums took twice as long (uncoalesced loads, cells of unlike
+// size in a warp: 63,517 tetrahedra at 100 a cell 341 -> 168 us, 48,640 hexahedra
+// at 50 116 -> 55 us, steps 11-20 from the freestream).
 constexpr int kOrderedWarps = 4;
 constexpr int kOrderedGroup = 32;
 

@@ -177,7 +177,10 @@ void dsmc_default_params(DsmcCaseParams* p);
  * patches (rebuildBoundaryEmitCache, src/ProcessDSMC.cpp:583-768), and
  * allocates all device state. Replaces ProcessDSMC::ProcessDSMC
  * (src/ProcessDSMC.cpp:271-288) plus Collision_constant_initial
- * (src/MeshparticalInitial.cpp:798-810). device < 0 uses the current one. */
+ * (src/MeshparticalInitial.cpp:798-810). device < 0 uses the current one.
+ * The handle holds, besides the particles (72 bytes each in mixed precision, 128
+ * in FP64, of its capacity), up to about 5 KB of device memory per cell and in mixed
+ * precision 6 MB for transfers. */
 int dsmc_create(const DsmcMeshDesc* mesh, const DsmcMeshMessage* mess,
                 const DsmcCaseParams* params, int device, DsmcHandle** out);
 
@@ -329,7 +332,10 @@ int dsmc_get_counters(DsmcHandle* h, DsmcCounters* out);
  * re-emitted. Outputs (any may be NULL): final cell (-1 removed/dropped),
  * ifout (0 stayed, 1 crossed, -1 removed/dropped), first non-interface face
  * and its triangle tag (-1/0 if none), number of crossings, final position,
- * velocity and remaining dt. Runs at the handle's precision. */
+ * velocity and remaining dt. Runs at the handle's precision. The handle keeps the
+ * call's device memory, 140 bytes per particle of the largest call up to
+ * 131,072 (18 MB), for the next; a call that needs more than it has allocates
+ * it. */
 int dsmc_trace(DsmcHandle* h, int64_t n,
                const double* px, const double* py, const double* pz,
                const double* vx, const double* vy, const double* vz,
@@ -391,7 +397,7 @@ int dsmc_sync(DsmcHandle* h);
 typedef struct DsmcLaunchShape {
     int32_t move_threads;          /* threads per block of the move kernel: 128 or 256 */
     int32_t move_blocks_per_sm;    /* move grid = SMs x this, 1..32 (particles per thread follow) */
-    int32_t sort_blocks_per_sm;    /* rank / scatter / gather grids = SMs x this, 1..32 */
+    int32_t sort_blocks_per_sm;    /* scatter / gather grids = SMs x this, 1..32 (the rank pass: at most 5, one wave) */
     int32_t collide_blocks_per_sm; /* cap on the collision grid per SM, 1..32 (at most the resident blocks; default 32) */
     int32_t stay_per_thread;       /* particles per thread of the move's stay pass: 1, 2 or 4 (default 4) */
 } DsmcLaunchShape;
@@ -403,8 +409,9 @@ int dsmc_set_launch_shape(DsmcHandle* h, const DsmcLaunchShape* shape);
 /* Runs full steps first_istep, first_istep+1, ... of the case, timing each
  * stage, and keeps per stage the fastest of a few shapes (move: block size
  * x blocks per SM, particles per thread of the stay pass; sort: blocks per
- * SM; collide keeps its cap). The steps
- * are ordinary steps of the case (about 15 x trial_steps of them);
+ * SM; collide keeps its cap). Timed steps run the stages one after another, so
+ * the move is timed without the injection that runs beside it otherwise. The
+ * steps are ordinary steps of the case (about 15 x trial_steps of them);
  * *next_istep receives the next step to run, *chosen the shape kept. */
 int dsmc_autotune(DsmcHandle* h, int32_t first_istep, int32_t trial_steps, int32_t* next_istep,
                   DsmcLaunchShape* chosen);
