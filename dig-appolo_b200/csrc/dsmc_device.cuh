@@ -109,13 +109,13 @@ struct DevConsts {
     double expLB;        // 1 / (2.5 - omega): Larsen-Borgnakke energy-fraction exponent
     double invAlpha;     // 1 / alpha: VSS scattering exponent
     float vhsExpF;       // 1 - 2 eta: exponent of the VHS sigma*c ratio (FP32 path)
-    float vhsHalfF;      // half of it where the FP64 acceptance may be settled in FP32, else NaN (pair_accept)
     float prelaxF;       // P_relax (FP32 path)
     float invPrelaxF;    // 1 / P_relax, 0 when P_relax is 0 (FP32 path)
     uint32_t seedLo, seedHi;
     int maxCross;
     int nss, nscheme, nevery, nrepeat;
     int wallStats;
+    float vhsHalfF;      // (1 - 2 eta) / 2 where the FP64 acceptance may be settled in FP32, else NaN (pair_accept)
 };
 
 // ---------------------------------------------------------------------------
