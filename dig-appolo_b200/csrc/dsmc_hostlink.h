@@ -9,17 +9,17 @@
 // device or a gather on the host, is the caller's. A transfer allocates no
 // device memory.
 //
-// The blocks, 6 MB, are freed with the handle. They are ordinary memory for
-// the first kPlain bytes that a handle moves and page-locked after that, since
-// page-locking them takes 2.6 to 7.5 ms: a handle that moves little (a few
-// tracing checks, a small restart) does without, and one that moves more has
-// by then gained about as much over the transfers it replaces. First tracing
-// check on a handle, 5,000 / 50,000 / 200,000 particles on 6,080 cells: 0.6 / 3.1 /
-// 9.6 ms (page-locked at once 8.3 / 9.2 / 13.4; a copy per column and array
-// 1.3 / 4.0 / 14.3), later ones 0.3 / 1.4 / 4.8. With kPlain at 16 MB, checks of
-// 50,000 were behind the copies by column until the sixth. Where none can be
-// page-locked, ordinary memory does for good (the copies then wait for each
-// other).
+// A thread's two blocks (1 MB; 6 MB for all) are page-locked when a transfer
+// first gives the thread work, and given back with the handle: 0.4 ms for one
+// thread's, 1 to 2.5 for all (cudaHostRegister; cudaHostAlloc of all 6 MB took
+// 2.6 to 7.5, whatever the transfer). A handle's first kPlain transfers of no
+// more than kPlainItems values use them as ordinary memory: the one or two
+// tracing checks of some particles that a program may make. First tracing
+// check on a handle, 1 / 5,000 / 50,000 / 200,000 particles on 6,080 cells: 0.4 /
+// 0.7 / 3.6 / 8.0 ms, with all blocks page-locked at once 7.4 / 7.5 / 9.5 / 13.6, with
+// a copy per column and array 0.5 / 1.4 / 4.1 / 15; from the fourth on, on every
+// way but the last, 0.2 / 0.4 / 1.5 / 4.6. Blocks that cannot be page-locked stay
+// ordinary memory (their copies then wait).
 #pragma once
 
 #include <algorithm>
@@ -36,14 +36,16 @@ struct HostLink {
     static constexpr int kSlots = 2 * kThreads;
     static constexpr int64_t kItems = 65536;
     static constexpr size_t kBytes = (size_t)kItems * 8;   // of a block: values of at most 8 bytes
-
-    static constexpr int64_t kPlain = 32 << 20;
+    static constexpr size_t kPage = 4096;
+    static constexpr int kPlain = 6;
+    static constexpr int64_t kPlainItems = 4 * kItems;
 
     int device = 0;                  // set by the owner
     cudaStream_t stream = nullptr;
     char* blocks = nullptr;          // [kSlots][kBytes]
-    bool pinned = false;             // whether they are page-locked
-    int64_t plainLeft = kPlain;      // bytes still to be moved through ordinary memory
+    int ready = 0;                   // threads whose blocks have been page-locked (or could not be)
+    bool pinned[kThreads] = {};      // page-locked in one call from this thread's blocks on
+    int plain = 0;                   // small transfers so far
     char* staged = nullptr;          // the same on the device, for values converted there (the caller's)
     cudaEvent_t event[kSlots] = {};
 
@@ -55,32 +57,14 @@ struct HostLink {
         char* dev;
     };
 
-    // Makes the blocks ready for a transfer of `bytes`.
-    cudaError_t ready(int64_t bytes)
-    {
-        if (bytes <= plainLeft) {
-            plainLeft -= bytes;
-        } else if (!pinned && plainLeft >= 0) {
-            plainLeft = -1;
-            void* q = nullptr;
-            if (cudaHostAlloc(&q, kSlots * kBytes, cudaHostAllocDefault) == cudaSuccess) {
-                freeBlocks();
-                blocks = static_cast<char*>(q);
-                pinned = true;
-            } else {
-                (void)cudaGetLastError();
-            }
-        }
-        if (!blocks && !(blocks = static_cast<char*>(std::malloc(kSlots * kBytes)))) return cudaErrorMemoryAllocation;
-        cudaError_t e = cudaSuccess;
-        for (cudaEvent_t& ev : event)
-            if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-        if (e != cudaSuccess) (void)cudaGetLastError();   // reported here, not by a later launch
-        return e;
-    }
     void release()
     {
-        freeBlocks();
+        if (blocks) cudaStreamSynchronize(stream);   // copies that a failed transfer left
+        for (int t = 0; t < kThreads; ++t)
+            if (pinned[t]) { cudaHostUnregister(blocks + 2 * t * kBytes); pinned[t] = false; }
+        std::free(blocks);
+        blocks = nullptr;
+        ready = 0;
         for (cudaEvent_t& ev : event)
             if (ev) { cudaEventDestroy(ev); ev = nullptr; }
     }
@@ -126,14 +110,29 @@ struct HostLink {
     }
 
 private:
-    void freeBlocks()
+    // Blocks and events for a transfer of `items` values by `threads` threads.
+    cudaError_t prepare(int64_t items, int threads)
     {
-        for (cudaEvent_t ev : event)
-            if (ev) cudaEventSynchronize(ev);   // the copies that read or write them
-        if (pinned) cudaFreeHost(blocks);
-        else std::free(blocks);
-        blocks = nullptr;
-        pinned = false;
+        if (!blocks && !(blocks = static_cast<char*>(std::aligned_alloc(kPage, kSlots * kBytes))))
+            return cudaErrorMemoryAllocation;
+        for (int s = 0; s < 2 * threads; ++s)
+            if (!event[s]) {
+                const cudaError_t e = cudaEventCreateWithFlags(&event[s], cudaEventDisableTiming);
+                if (e != cudaSuccess) {
+                    (void)cudaGetLastError();   // reported here, not by a later launch
+                    return e;
+                }
+            }
+        if (threads <= ready) return cudaSuccess;
+        if (items <= kPlainItems && plain < kPlain) {
+            ++plain;
+            return cudaSuccess;
+        }
+        pinned[ready] = cudaHostRegister(blocks + 2 * ready * kBytes, 2 * (threads - ready) * kBytes,
+                                         cudaHostRegisterDefault) == cudaSuccess;
+        if (!pinned[ready]) (void)cudaGetLastError();
+        ready = threads;
+        return cudaSuccess;
     }
 
     // step(slot, block) for every block, a thread's two slots in turn, and at
@@ -147,7 +146,11 @@ private:
             items += n[c];
         }
         if (total == 0) return cudaSuccess;
-        if (const cudaError_t e = ready(items * 8)) return e;
+        const int hw = (int)std::thread::hardware_concurrency();
+        // a thread for every block of values there are (starting one costs
+        // about what a block does)
+        const int threads = (int)std::max<int64_t>(1, std::min<int64_t>(items / kItems, std::min(kThreads, hw > 0 ? hw : 1)));
+        if (const cudaError_t e = prepare(items, threads)) return e;
         std::atomic<int64_t> next{0};
         std::atomic<int> error{0};
         auto work = [&](int t) {
@@ -168,10 +171,6 @@ private:
             for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = step(2 * t + (b ^ i), nullptr);
             if (e != cudaSuccess) error.store((int)e);
         };
-        const int hw = (int)std::thread::hardware_concurrency();
-        // a thread for every block of values there are (starting one costs
-        // about what a block does)
-        const int threads = (int)std::min<int64_t>(items / kItems, std::min(kThreads, hw > 0 ? hw : 1));
         std::thread pool[kThreads];
         for (int t = 1; t < threads; ++t) {
             try {

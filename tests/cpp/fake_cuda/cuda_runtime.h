@@ -1,6 +1,6 @@
 // The few CUDA runtime calls of csrc/dsmc_hostlink.h on the host, counted, for
-// a CPU test of it: copies are done when they are issued, page-locked memory
-// is ordinary memory, and its allocation can be made to fail.
+// a CPU test of it: copies are done when they are issued, page-locking
+// changes nothing, and can be made to fail.
 #pragma once
 
 #include <atomic>
@@ -11,11 +11,13 @@
 enum cudaError_t { cudaSuccess = 0, cudaErrorInvalidValue = 1, cudaErrorMemoryAllocation = 2 };
 typedef struct FakeStream* cudaStream_t;
 typedef struct FakeEvent* cudaEvent_t;
-enum { cudaHostAllocDefault = 0, cudaEventDisableTiming = 2 };
+enum { cudaHostRegisterDefault = 0, cudaEventDisableTiming = 2 };
 
 namespace fake {
-inline bool failHostAlloc = false;
-inline std::atomic<int> hostAllocs{0}, hostFrees{0}, events{0};
+inline bool failRegister = false;
+inline int registered = 0;
+inline size_t registeredBytes = 0;
+inline std::atomic<int> events{0};
 inline cudaError_t lastError = cudaSuccess;
 }  // namespace fake
 
@@ -26,19 +28,19 @@ inline cudaError_t cudaGetLastError()
     fake::lastError = cudaSuccess;
     return e;
 }
-inline cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
+inline cudaError_t cudaHostRegister(void* p, size_t n, unsigned)
 {
-    if (fake::failHostAlloc) return fake::lastError = cudaErrorMemoryAllocation;
-    ++fake::hostAllocs;
-    *p = std::malloc(n);
+    if (fake::failRegister || !p || !n) return fake::lastError = cudaErrorMemoryAllocation;
+    ++fake::registered;
+    fake::registeredBytes += n;
     return cudaSuccess;
 }
-inline cudaError_t cudaFreeHost(void* p)
+inline cudaError_t cudaHostUnregister(void* p)
 {
-    ++fake::hostFrees;
-    std::free(p);
-    return cudaSuccess;
+    --fake::registered;
+    return p ? cudaSuccess : cudaErrorInvalidValue;
 }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 inline cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned)
 {
     *e = reinterpret_cast<cudaEvent_t>(std::malloc(1));

@@ -50,34 +50,38 @@ bool round_trip(HostLink& L, int64_t n, int salt)
 
 int main()
 {
+    constexpr int64_t K = HostLink::kItems;
     for (bool fail : {false, true}) {
-        fake::failHostAlloc = fail;
-        fake::hostAllocs = fake::hostFrees = 0;
-        {
-            HostLink L;
-            check(L.in(0, nullptr, [](const HostLink::Block&) {}, [](const HostLink::Block&) { return cudaSuccess; }) ==
-                          cudaSuccess && !L.blocks, "no columns, no memory", 0);
-            int64_t moved = 0;
-            int salt = 0;
-            const int64_t sizes[] = {1, 2, HostLink::kItems - 1, HostLink::kItems, HostLink::kItems + 1, 5 * HostLink::kItems + 3};
-            for (int round = 0; round < 4; ++round)
-                for (int64_t n : sizes) {
-                    const int64_t one = (n + n / 2 + n + 1) * 8;
-                    check(round_trip(L, n, ++salt), "values", n);
-                    moved += 2 * one;
-                    if (moved <= HostLink::kPlain) check(fake::hostAllocs == 0, "page-locked early", moved);
-                }
-            check(moved > HostLink::kPlain, "the sizes go past the ordinary blocks", moved);
-            check(fake::hostAllocs == (fail ? 0 : 1) && L.pinned == !fail, "page-locked once", fake::hostAllocs);
-            check(fake::lastError == cudaSuccess, "no error left behind", fake::lastError);
-            // an error of a copy ends the transfer and leaves the link usable
-            const int64_t n = 3 * HostLink::kItems;
-            check(L.in(1, &n, [](const HostLink::Block&) {}, [](const HostLink::Block&) { return cudaErrorInvalidValue; }) ==
-                      cudaErrorInvalidValue, "the copy's error", n);
-            check(round_trip(L, 1000, 99), "values after an error", 1000);
-            L.release();
-        }
-        check(fake::hostFrees == fake::hostAllocs && fake::events == 0, "given back", fake::hostFrees);
+        fake::failRegister = fail;
+        fake::registeredBytes = 0;
+        HostLink L;
+        check(L.in(0, nullptr, [](const HostLink::Block&) {}, [](const HostLink::Block&) { return cudaSuccess; }) ==
+                      cudaSuccess && !L.blocks, "no columns, no memory", 0);
+        // kPlain small transfers without page-locking, then a thread's blocks
+        int salt = 0;
+        for (int k = 0; k < HostLink::kPlain / 2; ++k) check(round_trip(L, 1 + 7 * k, ++salt), "values", k);
+        check(fake::registeredBytes == 0 && fake::lastError == cudaSuccess, "page-locked early", 0);
+        check(round_trip(L, 5, ++salt), "values", 5);
+        check(fake::registeredBytes == (fail ? 0 : 2 * HostLink::kBytes), "one thread's blocks", (long long)fake::registeredBytes);
+        for (int round = 0; round < 2; ++round)
+            for (int64_t n : {int64_t(1), K / 3, K - 1, K, K + 1, 2 * K + 5, 5 * K + 3, int64_t(100)})
+                check(round_trip(L, n, ++salt), "values", n);
+        check(fake::registeredBytes <= HostLink::kSlots * HostLink::kBytes, "each block once", (long long)fake::registeredBytes);
+        check(fake::lastError == cudaSuccess, "no error left behind", fake::lastError);
+        // an error of a copy ends the transfer and leaves the link usable
+        const int64_t n = 3 * K;
+        check(L.in(1, &n, [](const HostLink::Block&) {}, [](const HostLink::Block&) { return cudaErrorInvalidValue; }) ==
+                  cudaErrorInvalidValue, "the copy's error", n);
+        check(round_trip(L, 1000, ++salt), "values after an error", 1000);
+        L.release();
+        check(fake::registered == 0 && fake::events == 0 && !L.blocks, "given back", fake::registered);
+        // a large first transfer page-locks at once, what it needs
+        fake::registeredBytes = 0;
+        check(round_trip(L, 6 * K, ++salt), "values", 6 * K);
+        check(fail || (fake::registeredBytes >= 2 * HostLink::kBytes &&
+                       fake::registeredBytes <= HostLink::kSlots * HostLink::kBytes), "page-locked", (long long)fake::registeredBytes);
+        L.release();
+        check(fake::registered == 0 && fake::events == 0, "given back", fake::registered);
     }
     if (failures) return 1;
     std::printf("ok\n");

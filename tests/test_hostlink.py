@@ -1,8 +1,9 @@
 """The blocks of host memory that transfers pass through
 (csrc/dsmc_hostlink.h), on the CPU with a stand-in for the CUDA runtime
 (tests/cpp/fake_cuda): values at the ends of a block, through ordinary and
-page-locked memory and where none can be page-locked; nothing is page-locked
-for a handle's first 32 MB."""
+page-locked memory and where none can be page-locked; a handle's first small
+transfers page-lock nothing, and the others the blocks of the threads they
+use."""
 import os
 import shutil
 import subprocess
