@@ -9,17 +9,18 @@
 // device or a gather on the host, is the caller's. A transfer allocates no
 // device memory.
 //
-// A thread's two blocks (1 MB; 6 MB for all) are page-locked when a transfer
-// first gives the thread work, and given back with the handle: 0.4 ms for one
-// thread's, 1 to 2.5 for all (cudaHostRegister; cudaHostAlloc of all 6 MB took
-// 2.6 to 7.5, whatever the transfer). A handle's first kPlain transfers of no
-// more than kPlainItems values use them as ordinary memory: the one or two
-// tracing checks of some particles that a program may make. First tracing
-// check on a handle, 1 / 5,000 / 50,000 / 200,000 particles on 6,080 cells: 0.4 /
-// 0.7 / 3.6 / 8.0 ms, with all blocks page-locked at once 7.4 / 7.5 / 9.5 / 13.6, with
-// a copy per column and array 0.5 / 1.4 / 4.1 / 15; from the fourth on, on every
-// way but the last, 0.2 / 0.4 / 1.5 / 4.6. Blocks that cannot be page-locked stay
-// ordinary memory (their copies then wait).
+// The blocks, 1 MB a thread, are page-locked two threads' at a time when a
+// transfer first gives those threads work, and given back with the handle. They
+// lie in huge pages where the system gives any, one for two threads:
+// page-locking one takes 0.4 to 0.7 ms, all three 0.6 to 1.4; in small pages 1 to 2.6
+// and 2 to 7, and cudaHostAlloc of all 6 MB as much. A handle's first kPlain
+// transfers of no more than one block's values, the one or two tracing checks of
+// a few particles that a program may make, go through ordinary memory instead.
+// First tracing check on a handle, 1 / 5,000 / 50,000 / 200,000 particles on 6,080
+// cells: 0.4 / 0.7 / 3.4 / 7.8 ms, where all blocks allocated at once took 8.1 / 7.8 /
+// 10 / 14, and a copy per column and array 0.5 / 1.3 / 3.9 / 14; later ones 0.2 / 0.4 /
+// 1.5 / 4.6. Blocks that cannot be page-locked stay ordinary memory (their copies
+// then wait).
 #pragma once
 
 #include <algorithm>
@@ -27,6 +28,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <thread>
 
 namespace dsmc {
@@ -36,16 +38,19 @@ struct HostLink {
     static constexpr int kSlots = 2 * kThreads;
     static constexpr int64_t kItems = 65536;
     static constexpr size_t kBytes = (size_t)kItems * 8;   // of a block: values of at most 8 bytes
-    static constexpr size_t kPage = 4096;
+    static constexpr size_t kHuge = 2 << 20;               // a huge page: the blocks of kUnit threads
+    static constexpr int kUnit = (int)(kHuge / (2 * kBytes));
     static constexpr int kPlain = 6;
-    static constexpr int64_t kPlainItems = 4 * kItems;
+    static_assert(kUnit >= 1 && kThreads % kUnit == 0, "whole huge pages");
 
     int device = 0;                  // set by the owner
     cudaStream_t stream = nullptr;
-    char* blocks = nullptr;          // [kSlots][kBytes]
+    void* mapped = nullptr;          // kSlots * kBytes + kHuge
+    char* blocks = nullptr;          // [kSlots][kBytes] in there, from a huge page's start
     int ready = 0;                   // threads whose blocks have been page-locked (or could not be)
     bool pinned[kThreads] = {};      // page-locked in one call from this thread's blocks on
     int plain = 0;                   // small transfers so far
+    char* small = nullptr;           // [2][kBytes], theirs
     char* staged = nullptr;          // the same on the device, for values converted there (the caller's)
     cudaEvent_t event[kSlots] = {};
 
@@ -59,11 +64,13 @@ struct HostLink {
 
     void release()
     {
-        if (blocks) cudaStreamSynchronize(stream);   // copies that a failed transfer left
+        if (blocks || small) cudaStreamSynchronize(stream);   // copies that a failed transfer left
         for (int t = 0; t < kThreads; ++t)
             if (pinned[t]) { cudaHostUnregister(blocks + 2 * t * kBytes); pinned[t] = false; }
-        std::free(blocks);
-        blocks = nullptr;
+        if (mapped) munmap(mapped, kSlots * kBytes + kHuge);
+        std::free(small);
+        mapped = nullptr;
+        blocks = small = nullptr;
         ready = 0;
         for (cudaEvent_t& ev : event)
             if (ev) { cudaEventDestroy(ev); ev = nullptr; }
@@ -110,11 +117,9 @@ struct HostLink {
     }
 
 private:
-    // Blocks and events for a transfer of `items` values by `threads` threads.
-    cudaError_t prepare(int64_t items, int threads)
+    // Blocks (at *at) and events for a transfer of `items` values by `threads` threads.
+    cudaError_t prepare(int64_t items, int threads, char** at)
     {
-        if (!blocks && !(blocks = static_cast<char*>(std::aligned_alloc(kPage, kSlots * kBytes))))
-            return cudaErrorMemoryAllocation;
         for (int s = 0; s < 2 * threads; ++s)
             if (!event[s]) {
                 const cudaError_t e = cudaEventCreateWithFlags(&event[s], cudaEventDisableTiming);
@@ -123,15 +128,30 @@ private:
                     return e;
                 }
             }
-        if (threads <= ready) return cudaSuccess;
-        if (items <= kPlainItems && plain < kPlain) {
+        if (ready == 0 && items <= kItems && plain < kPlain) {
             ++plain;
-            return cudaSuccess;
+            if (!small) small = static_cast<char*>(std::malloc(2 * kBytes));
+            *at = small;
+            return small ? cudaSuccess : cudaErrorMemoryAllocation;
         }
-        pinned[ready] = cudaHostRegister(blocks + 2 * ready * kBytes, 2 * (threads - ready) * kBytes,
-                                         cudaHostRegisterDefault) == cudaSuccess;
-        if (!pinned[ready]) (void)cudaGetLastError();
-        ready = threads;
+        if (!blocks) {
+            void* q = mmap(nullptr, kSlots * kBytes + kHuge, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+            if (q == MAP_FAILED) return cudaErrorMemoryAllocation;
+            mapped = q;
+            blocks = static_cast<char*>(q) + (kHuge - (uintptr_t)q % kHuge) % kHuge;
+            (void)madvise(blocks, kSlots * kBytes, MADV_HUGEPAGE);
+            // a fork must not make the pages copy-on-write: this process's next
+            // write would move them away from where the device was told they are
+            (void)madvise(blocks, kSlots * kBytes, MADV_DONTFORK);
+        }
+        if (threads > ready) {
+            const int upTo = std::min(kThreads, (threads + kUnit - 1) / kUnit * kUnit);
+            pinned[ready] = cudaHostRegister(blocks + 2 * ready * kBytes, 2 * (upTo - ready) * kBytes,
+                                             cudaHostRegisterDefault) == cudaSuccess;
+            if (!pinned[ready]) (void)cudaGetLastError();
+            ready = upTo;
+        }
+        *at = blocks;
         return cudaSuccess;
     }
 
@@ -150,7 +170,8 @@ private:
         // a thread for every block of values there are (starting one costs
         // about what a block does)
         const int threads = (int)std::max<int64_t>(1, std::min<int64_t>(items / kItems, std::min(kThreads, hw > 0 ? hw : 1)));
-        if (const cudaError_t e = prepare(items, threads)) return e;
+        char* at = nullptr;
+        if (const cudaError_t e = prepare(items, threads, &at)) return e;
         std::atomic<int64_t> next{0};
         std::atomic<int> error{0};
         auto work = [&](int t) {
@@ -164,7 +185,7 @@ private:
                 k.off = q * kItems;
                 k.len = std::min(kItems, n[k.col] - k.off);
                 const int slot = 2 * t + b;
-                k.host = blocks + (size_t)slot * kBytes;
+                k.host = at + (size_t)slot * kBytes;
                 k.dev = staged + (size_t)slot * kBytes;
                 e = step(slot, &k);
             }

@@ -6,6 +6,8 @@
 #include "dsmc_hostlink.h"
 
 #include <cstdio>
+#include <fstream>
+#include <string>
 #include <vector>
 
 using dsmc::HostLink;
@@ -46,6 +48,20 @@ bool round_trip(HostLink& L, int64_t n, int salt)
     return in == cudaSuccess && out == cudaSuccess && dev == src && back == src;
 }
 
+// whether the mapping at p is left out of a fork
+bool not_forked(const void* p)
+{
+    std::ifstream maps("/proc/self/smaps");
+    std::string line;
+    bool in = false;
+    while (std::getline(maps, line)) {
+        unsigned long a = 0, b = 0;
+        if (std::sscanf(line.c_str(), "%lx-%lx ", &a, &b) == 2) in = (unsigned long)p >= a && (unsigned long)p < b;
+        if (in && line.compare(0, 8, "VmFlags:") == 0) return line.find(" dc") != std::string::npos;
+    }
+    return false;
+}
+
 }  // namespace
 
 int main()
@@ -57,15 +73,16 @@ int main()
         HostLink L;
         check(L.in(0, nullptr, [](const HostLink::Block&) {}, [](const HostLink::Block&) { return cudaSuccess; }) ==
                       cudaSuccess && !L.blocks, "no columns, no memory", 0);
-        // kPlain small transfers without page-locking, then a thread's blocks
+        // kPlain small transfers without page-locking, then what a thread needs
         int salt = 0;
         for (int k = 0; k < HostLink::kPlain / 2; ++k) check(round_trip(L, 1 + 7 * k, ++salt), "values", k);
         check(fake::registeredBytes == 0 && fake::lastError == cudaSuccess, "page-locked early", 0);
         check(round_trip(L, 5, ++salt), "values", 5);
-        check(fake::registeredBytes == (fail ? 0 : 2 * HostLink::kBytes), "one thread's blocks", (long long)fake::registeredBytes);
+        check(fake::registeredBytes == (fail ? 0 : HostLink::kHuge), "one huge page", (long long)fake::registeredBytes);
         for (int round = 0; round < 2; ++round)
             for (int64_t n : {int64_t(1), K / 3, K - 1, K, K + 1, 2 * K + 5, 5 * K + 3, int64_t(100)})
                 check(round_trip(L, n, ++salt), "values", n);
+        check(not_forked(L.blocks) && not_forked(L.blocks + HostLink::kSlots * HostLink::kBytes - 1), "left out of a fork", 0);
         check(fake::registeredBytes <= HostLink::kSlots * HostLink::kBytes, "each block once", (long long)fake::registeredBytes);
         check(fake::lastError == cudaSuccess, "no error left behind", fake::lastError);
         // an error of a copy ends the transfer and leaves the link usable
@@ -78,7 +95,7 @@ int main()
         // a large first transfer page-locks at once, what it needs
         fake::registeredBytes = 0;
         check(round_trip(L, 6 * K, ++salt), "values", 6 * K);
-        check(fail || (fake::registeredBytes >= 2 * HostLink::kBytes &&
+        check(fail || (fake::registeredBytes >= HostLink::kHuge &&
                        fake::registeredBytes <= HostLink::kSlots * HostLink::kBytes), "page-locked", (long long)fake::registeredBytes);
         L.release();
         check(fake::registered == 0 && fake::events == 0, "given back", fake::registered);

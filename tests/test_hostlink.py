@@ -3,7 +3,7 @@
 (tests/cpp/fake_cuda): values at the ends of a block, through ordinary and
 page-locked memory and where none can be page-locked; a handle's first small
 transfers page-lock nothing, and the others the blocks of the threads they
-use."""
+use; the blocks are left out of a fork."""
 import os
 import shutil
 import subprocess
